@@ -44,6 +44,21 @@ __device__ __forceinline__ float2 fsub2(float2 a, float2 b) {
     return *reinterpret_cast<float2*>(&d);
 }
 
+__device__ __forceinline__ float2 fmul2(float2 a, float2 b) {
+    uint64_t d;
+    asm("mul.rn.f32x2 %0, %1, %2;"
+        : "=l"(d)
+        : "l"(*reinterpret_cast<const uint64_t*>(&a)), "l"(*reinterpret_cast<const uint64_t*>(&b)));
+    return *reinterpret_cast<float2*>(&d);
+}
+__device__ __forceinline__ float2 fadd2(float2 a, float2 b) {
+    uint64_t d;
+    asm("add.rn.f32x2 %0, %1, %2;"
+        : "=l"(d)
+        : "l"(*reinterpret_cast<const uint64_t*>(&a)), "l"(*reinterpret_cast<const uint64_t*>(&b)));
+    return *reinterpret_cast<float2*>(&d);
+}
+
 // (float)(1.0 / (double)x): the reference computes these reciprocals in
 // double and rounds once to float (inc/utils/space.hpp:760,774;
 // inc/index/HASearcher.hpp:56).

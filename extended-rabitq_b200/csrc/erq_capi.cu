@@ -41,6 +41,7 @@
 #include "order.cuh"
 #include "scan.cuh"
 #include "scan_batch.cuh"
+#include "scan_mma.cuh"
 
 using namespace erq;
 
@@ -646,20 +647,20 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
     return fn;
 }
 
-// 2-D map of a row-major BF16 matrix [rows][cols]: boxes of 64 columns
-// (128 bytes, the swizzle span) by box_rows rows, 128-byte swizzle, zero fill
-// outside the matrix.
-erq_status tensor_map_bf16(CUtensorMap* m, const void* ptr, uint64_t rows, uint64_t cols,
-                           uint32_t box_rows) {
+// 2-D map of a row-major matrix [rows][cols] of elt-byte elements: boxes of
+// box_cols columns (128 bytes, the swizzle span) by box_rows rows, 128-byte
+// swizzle, zero fill outside the matrix.
+erq_status tensor_map_2d(CUtensorMap* m, CUtensorMapDataType type, uint64_t elt, const void* ptr,
+                         uint64_t rows, uint64_t cols, uint32_t box_cols, uint32_t box_rows) {
     auto fn = tensor_map_encoder();
     if (!fn) return fail(ERQ_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
-    if ((reinterpret_cast<uintptr_t>(ptr) & 15) || (cols * 2) % 16)
+    if ((reinterpret_cast<uintptr_t>(ptr) & 15) || (cols * elt) % 16)
         return fail(ERQ_ERR_INVALID_ARGUMENT, "TMA operand not 16-byte aligned");
     cuuint64_t dims[2] = {cols, rows};
-    cuuint64_t strides[1] = {cols * 2};
-    cuuint32_t box[2] = {64, box_rows};
+    cuuint64_t strides[1] = {cols * elt};
+    cuuint32_t box[2] = {box_cols, box_rows};
     cuuint32_t estr[2] = {1, 1};
-    CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box,
+    CUresult r = fn(m, type, 2, const_cast<void*>(ptr), dims, strides, box,
                     estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                     CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return fail(ERQ_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", (int)r);
@@ -677,8 +678,9 @@ erq_status gemm_tc(const __nv_bfloat16* A, const __nv_bfloat16* B, float* C, int
     if (M <= 0 || N <= 0) return ERQ_OK;
     if (Kd <= 0 || Kd % kTcBK) return fail(ERQ_ERR_INVALID_ARGUMENT, "GEMM depth %d not a multiple of 64", Kd);
     CUtensorMap ta, tb;
-    ERQ_TRY(tensor_map_bf16(&ta, A, (uint64_t)M, (uint64_t)Kd, kTcBM));
-    ERQ_TRY(tensor_map_bf16(&tb, B, (uint64_t)N, (uint64_t)Kd, kTcBN));
+    constexpr auto kBf16 = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
+    ERQ_TRY(tensor_map_2d(&ta, kBf16, 2, A, (uint64_t)M, (uint64_t)Kd, kTcBK, kTcBM));
+    ERQ_TRY(tensor_map_2d(&tb, kBf16, 2, B, (uint64_t)N, (uint64_t)Kd, kTcBK, kTcBN));
     uint32_t* status = nullptr;
     ERQ_TRY(tc_status_ptr(&status));
     {
@@ -727,6 +729,9 @@ struct Batch {
     uint32_t* order_pairs = nullptr;  // [nq * nprobe]
     uint32_t* order_q = nullptr;      // [nq]
     float* bmin = nullptr;            // smallest lower bound per scanned block (S / 32 entries)
+    uint8_t* qrows = nullptr;         // [2][nq * nprobe][mma_row_bytes] quantized pairs (scan_mma.cuh)
+    uint32_t* item_off = nullptr;     // [K + 1] first work item of each cluster (scan_batch.cuh)
+    uint32_t* item_counter = nullptr; // the next work item
     uint32_t* fb_flag = nullptr;      // [nq] queries whose probe needs all K exact distances
     uint64_t* sortbuf = nullptr;      // [nq][sort_cap] probe sort keys too many for shared memory
     uint64_t sort_cap = 0;
@@ -771,8 +776,32 @@ uint64_t batch_queries(const erq_index* idx, uint64_t nprobe, uint64_t nq) {
     return std::min(b, nq);
 }
 
+// Whether a batch of at least `pairs` (query, probe) pairs scans on the tensor
+// cores (scan_mma.cuh).  Its products cost next to nothing per query, but a
+// batch pays for two more launches and the expansion of every probed block
+// whatever the number of queries that share it, while the lookups' cost grows
+// with pairs x dims.  Whole searches, lookups against products, us (best of
+// 3 x 10): 1M x 1536, K 4096: 64 pairs 479 / 483, 256 pairs 568 / 537, 1,024
+// pairs 824 / 732, 16,384 pairs 3,199 / 1,362; 768 dims, Zipf, K 4096: 1,024
+// pairs 1,697 / 1,687, 4,096 pairs 2,027 / 1,992; 128 dims, K 1024: 1,024
+// pairs 156 / 170, 4,096 pairs 201 / 196, 16,384 pairs 324 / 232.
+bool scan_mma_pays(const erq_index* idx, uint64_t pairs) {
+    return idx->factors == 1 && pairs >= 512 && pairs * idx->D >= (1ull << 20);
+}
+
+// Bytes of the quantized rows of nq * nprobe pairs, 0 when they are not kept:
+// when no batch of this size uses them (min_pairs: the pairs it has at
+// least), or when they would be more than the sums they lead to (S) and 1 GiB
+// - a very large batch over tiny clusters, which then scans by lookups.
+uint64_t mma_rows_bytes(const erq_index* idx, uint64_t nq, uint64_t nprobe, uint64_t min_pairs) {
+    if (!scan_mma_pays(idx, min_pairs) || nq * nprobe >= (1ull << 30)) return 0;
+    const uint64_t bytes = 2 * nq * nprobe * mma_row_bytes((int)idx->D);
+    return bytes <= std::max<uint64_t>(1ull << 30, nq * 128 * idx->top_blocks[nprobe]) ? bytes : 0;
+}
+
 template <class Alloc>
-erq_status alloc_batch(Alloc& s, const erq_index* idx, uint64_t nq, uint64_t nprobe, Batch& b) {
+erq_status alloc_batch(Alloc& s, const erq_index* idx, uint64_t nq, uint64_t nprobe, Batch& b,
+                       uint64_t min_pairs = 0) {
     b.nq = nq;
     ERQ_TRY(s.alloc(&b.dist, nq * idx->K));
     ERQ_TRY(s.alloc(&b.probe_cid, nq * nprobe));
@@ -786,14 +815,22 @@ erq_status alloc_batch(Alloc& s, const erq_index* idx, uint64_t nq, uint64_t npr
     ERQ_TRY(s.alloc(&b.qn, nq));
     ERQ_TRY(s.alloc(&b.keys, nq * nprobe));
     ERQ_TRY(s.alloc(&b.keys_q, nq));
-    ERQ_TRY(s.alloc(&b.buckets, 2 * (idx->K + 1)));
+    ERQ_TRY(s.alloc(&b.buckets, 3 * (idx->K + 1) + 1));
     b.buckets_q = b.buckets + idx->K + 1;
+    b.item_off = b.buckets_q + idx->K + 1;
+    b.item_counter = b.item_off + idx->K + 1;
     ERQ_TRY(s.alloc(&b.order_pairs, nq * nprobe));
     ERQ_TRY(s.alloc(&b.order_q, nq));
     ERQ_TRY(s.alloc(&b.bmin, nq * idx->top_blocks[nprobe]));
     ERQ_TRY(s.alloc(&b.fb_flag, nq));
     b.sort_cap = probe_sort_cap(idx, nprobe, true);
     if (b.sort_cap) ERQ_TRY(s.alloc(&b.sortbuf, nq * b.sort_cap));
+    // last: a batch whose rows do not fit the device scans by lookups instead
+    const uint64_t rows = mma_rows_bytes(idx, nq, nprobe, min_pairs);
+    if (rows && s.alloc(&b.qrows, rows) != ERQ_OK) {
+        b.qrows = nullptr;
+        cudaGetLastError();
+    }
     return ERQ_OK;
 }
 
@@ -1124,6 +1161,110 @@ erq_status launch_scan(const erq_index* idx, const Batch& b, uint64_t nprobe, cu
     return ERQ_OK;
 }
 
+// The work list of a batch's cluster-sorted pairs (scan_batch.cuh; order_both
+// with pairs_by_size false): items of up to QB queries and CB blocks, and the
+// arguments of the kernels that walk it.
+erq_status scan_work_list(const erq_index* idx, const Batch& b, uint64_t nprobe, int QB, int CB,
+                          ScanBatchArgs& a, cudaStream_t st) {
+    const int K = (int)idx->K;
+    {
+        LaunchTimer lt(kOrder, st);
+        scan_items_count_kernel<<<(unsigned)div_up(K, 256), 256, 0, st>>>(
+            b.buckets, idx->c_nblocks, idx->c_by_size, K, QB, CB, b.item_off);
+        lt.finish();
+    }
+    {
+        LaunchTimer lt(kOrder, st);
+        bucket_scan_kernel<<<1, kBucketScanThreads, 0, st>>>(b.item_off, b.item_off, (uint32_t)K + 1);
+        lt.finish();
+    }
+    ERQ_CUDA(cudaMemsetAsync(b.item_counter, 0, sizeof(uint32_t), st));
+    a = ScanBatchArgs{};
+    a.qrot = b.qrot;
+    a.centroids = idx->centroids;
+    a.probe_cid = b.probe_cid;
+    a.probe_sqy = b.probe_sqy;
+    a.codes = idx->codes;
+    a.c_first_block = idx->c_first_block;
+    a.c_nblocks = idx->c_nblocks;
+    a.s_off = b.s_off;
+    a.S = b.S;
+    a.qp_delta = b.delta;
+    a.qp_sumq = b.sumq;
+    a.onorm = idx->onorm;
+    a.c_size = idx->c_size;
+    a.bmin = b.bmin;
+    a.order_pairs = b.order_pairs;
+    a.bucket_end = b.buckets;
+    a.item_off = b.item_off;
+    a.c_order = idx->c_by_size;
+    a.item_counter = b.item_counter;
+    a.K = K;
+    a.D = (int)idx->D;
+    a.nprobe = (int)nprobe;
+    a.CB = CB;
+    return tc_status_ptr(&a.status);
+}
+
+// Blocks of a work item of scan_mma_kernel.  Scan time of the timed batches at
+// 8 / 16 / 32 / 64 / 256 blocks, us: 10,000 queries, nprobe 2, 1M x 1536: 588 /
+// 559 / 545 / 539 / 673; learned depths: 271 / 264 / 260 / 261 / 434; 2,000
+// queries, nprobe 64: 1,990 / 1,863 / 1,808 / 1,773 / 1,766; 64 queries, nprobe
+// 128, Zipf clusters: 148 / 144 / 144 / 158 / 302.
+constexpr int kMmaBlocksPerItem = 32;
+
+// The scan of a cluster-sorted batch on the tensor cores (scan_mma.cuh).
+erq_status launch_scan_mma(const erq_index* idx, const Batch& b, uint64_t nprobe, cudaStream_t st) {
+    const uint64_t pairs = b.nq * nprobe;
+    const int D = (int)idx->D;
+    {
+        static std::mutex mu;
+        static bool configured[kMaxDevices] = {};
+        int dev = 0;
+        ERQ_CUDA(cudaGetDevice(&dev));
+        std::lock_guard<std::mutex> g(mu);
+        if (!configured[dev]) {  // for every D
+            ERQ_CUDA(cudaFuncSetAttribute(scan_quantize_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int)quantize_smem_bytes(kMaxD)));
+            ERQ_CUDA(cudaFuncSetAttribute(scan_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int)mma_smem_bytes(kMaxD)));
+            configured[dev] = true;
+        }
+    }
+    {
+        QuantizeArgs z{};
+        z.qrot = b.qrot;
+        z.centroids = idx->centroids;
+        z.probe_cid = b.probe_cid;
+        z.probe_sqy = b.probe_sqy;
+        z.order_pairs = b.order_pairs;
+        z.bucket_end = b.buckets;
+        z.rows = b.qrows;
+        z.qp_delta = b.delta;
+        z.qp_sumq = b.sumq;
+        z.cap = pairs;
+        z.K = (int)idx->K;
+        z.D = D;
+        z.nprobe = (int)nprobe;
+        LaunchTimer t(kScan, st);
+        scan_quantize_kernel<<<(unsigned)div_up(pairs, kQuantizeWarps), kQuantizeWarps * 32,
+                               quantize_smem_bytes(D), st>>>(z);
+        t.finish();
+        ERQ_CUDA(cudaGetLastError());
+    }
+    ScanBatchArgs a{};
+    ERQ_TRY(scan_work_list(idx, b, nprobe, kMmaQueries, kMmaBlocksPerItem, a, st));
+    CUtensorMap rows;
+    ERQ_TRY(tensor_map_2d(&rows, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, b.qrows, 2 * pairs, mma_row_bytes(D), 128, 8));
+    const size_t smem = mma_smem_bytes(D);
+    const int per_sm = smem <= 112 * 1024 ? 2 : 1;
+    LaunchTimer t(kScan, st);
+    scan_mma_kernel<<<(unsigned)(device_sms() * per_sm), kMmaThreads, smem, st>>>(rows, (uint32_t)pairs, a);
+    t.finish();
+    ERQ_CUDA(cudaGetLastError());
+    return ERQ_OK;
+}
+
 // refine_warps: 4 or kWideWarps chooses the form; 0 takes the wide one when
 // the batch has no more queries than SMs.
 erq_status launch_refine(const erq_index* idx, const Batch& b, uint64_t nprobe, uint64_t k,
@@ -1229,6 +1370,21 @@ erq_status launch_refine(const erq_index* idx, const Batch& b, uint64_t nprobe, 
     return ERQ_OK;
 }
 
+// The work orders and the scan of a batch outside a plan; *ordered: b.order_q
+// holds the refinement's order.
+erq_status order_and_scan(const erq_index* idx, const Batch& b, uint64_t nprobe, cudaStream_t st,
+                          const int* q_nprobe, bool* ordered) {
+    if (b.qrows && scan_mma_pays(idx, q_nprobe ? b.nq : b.nq * nprobe)) {
+        ERQ_TRY(order_both(idx, b, nprobe, st, q_nprobe, false));
+        *ordered = true;
+        return launch_scan_mma(idx, b, nprobe, st);
+    }
+    erq_status oe;
+    *ordered = launch_order(idx, b, nprobe, st, q_nprobe, &oe);
+    ERQ_TRY(oe);
+    return launch_scan(idx, b, nprobe, st, q_nprobe, *ordered ? b.order_pairs : nullptr);
+}
+
 erq_status check_search_args(const erq_index* idx, uint64_t nq, uint64_t k, uint64_t nprobe,
                              const void* q, const void* ids) {
     if (!idx) return fail(ERQ_ERR_INVALID_ARGUMENT, "index is NULL");
@@ -1250,15 +1406,13 @@ erq_status search_device(const erq_index* idx, const float* qrot_dev, uint64_t n
     const uint64_t bq = batch_queries(idx, nprobe, nq);
     Scratch s(st, idx->pool);
     Batch b;
-    ERQ_TRY(alloc_batch(s, idx, bq, nprobe, b));
+    ERQ_TRY(alloc_batch(s, idx, bq, nprobe, b, bq * nprobe));
     for (uint64_t q0 = 0; q0 < nq; q0 += bq) {
         b.nq = std::min(bq, nq - q0);
         b.qrot = qrot_dev + q0 * idx->D;
         ERQ_TRY(launch_probe_tc(idx, b, nprobe, st));
-        erq_status oe;
-        const bool ordered = launch_order(idx, b, nprobe, st, nullptr, &oe);
-        ERQ_TRY(oe);
-        ERQ_TRY(launch_scan(idx, b, nprobe, st, nullptr, ordered ? b.order_pairs : nullptr));
+        bool ordered = false;
+        ERQ_TRY(order_and_scan(idx, b, nprobe, st, nullptr, &ordered));
         ERQ_TRY(launch_refine(idx, b, nprobe, k, ids_dev + q0 * k,
                               dists_dev ? dists_dev + q0 * k : nullptr, st, nullptr,
                               ordered ? b.order_q : nullptr));
@@ -2338,7 +2492,7 @@ static erq_status search_learned_entry(const erq_index* idx, const erq_probe_mod
     ERQ_TRY(s.alloc(&used, nq));
     const uint64_t bq = batch_queries(idx, nprobe_max, nq);
     Batch b;
-    ERQ_TRY(alloc_batch(s, idx, bq, nprobe_max, b));
+    ERQ_TRY(alloc_batch(s, idx, bq, nprobe_max, b, bq));
     ERQ_TRY(alloc_probe_lists(s, bq, b));
     float *near_d = nullptr, *feats = nullptr;
     ERQ_TRY(s.alloc(&near_d, bq * kFeatDists));
@@ -2362,10 +2516,8 @@ static erq_status search_learned_entry(const erq_index* idx, const erq_probe_mod
         ERQ_CUDA(cudaGetLastError());
         // exact distances only as deep as each query's chosen depth
         if (split) ERQ_TRY(launch_probe_finish(idx, b, nprobe_max, st, used + q0));
-        erq_status oe;
-        const bool ordered = launch_order(idx, b, nprobe_max, st, used + q0, &oe);
-        ERQ_TRY(oe);
-        ERQ_TRY(launch_scan(idx, b, nprobe_max, st, used + q0, ordered ? b.order_pairs : nullptr));
+        bool ordered = false;
+        ERQ_TRY(order_and_scan(idx, b, nprobe_max, st, used + q0, &ordered));
         ERQ_TRY(launch_refine(idx, b, nprobe_max, k, ids_out + q0 * k,
                               d_out ? d_out + q0 * k : nullptr, st, used + q0,
                               ordered ? b.order_q : nullptr));
@@ -2910,8 +3062,6 @@ struct erq_plan {
     float* near_d = nullptr;    // [max_batch][64]
     float* feats = nullptr;     // [max_batch][320]
     MlpWork wk;
-    uint32_t* item_off = nullptr;  // [K + 1]
-    uint32_t* counter = nullptr;
     cudaStream_t cap = nullptr;
     bool use_graphs = true;
     std::mutex mu;
@@ -2986,48 +3136,16 @@ bool tuning_valid(const erq_plan_tuning& t) {
            (t.refine_warps == 0 || t.refine_warps == 4 || t.refine_warps == (uint32_t)kWideWarps);
 }
 
-erq_status launch_scan_batched(erq_plan* p, uint64_t nq, const erq_plan_tuning& t, cudaStream_t st) {
-    const erq_index* idx = p->idx;
-    const int K = (int)idx->K;
-    {
-        LaunchTimer lt(kOrder, st);
-        scan_items_count_kernel<<<(unsigned)div_up(K, 256), 256, 0, st>>>(
-            p->b.buckets, idx->c_nblocks, idx->c_by_size, K, (int)t.queries_per_item,
-            (int)t.blocks_per_item, p->item_off);
-        lt.finish();
-    }
-    {
-        LaunchTimer lt(kOrder, st);
-        bucket_scan_kernel<<<1, kBucketScanThreads, 0, st>>>(p->item_off, p->item_off, (uint32_t)K + 1);
-        lt.finish();
-    }
-    ERQ_CUDA(cudaMemsetAsync(p->counter, 0, sizeof(uint32_t), st));
+// Whether the plan's batches of nq queries scan on the tensor cores (a learned
+// plan counts one pair per query, the least it can have).
+bool plan_scans_mma(const erq_plan* p, uint64_t nq) {
+    return p->b.qrows && scan_mma_pays(p->idx, p->model ? nq : nq * p->nprobe_run);
+}
+
+erq_status launch_scan_batched(erq_plan* p, const erq_plan_tuning& t, cudaStream_t st) {
+    if (plan_scans_mma(p, p->b.nq)) return launch_scan_mma(p->idx, p->b, p->nprobe_run, st);
     ScanBatchArgs a{};
-    a.qrot = p->b.qrot;
-    a.centroids = idx->centroids;
-    a.probe_cid = p->b.probe_cid;
-    a.probe_sqy = p->b.probe_sqy;
-    a.codes = idx->codes;
-    a.c_first_block = idx->c_first_block;
-    a.c_nblocks = idx->c_nblocks;
-    a.s_off = p->b.s_off;
-    a.S = p->b.S;
-    a.qp_delta = p->b.delta;
-    a.qp_sumq = p->b.sumq;
-    a.onorm = idx->onorm;
-    a.c_size = idx->c_size;
-    a.bmin = p->b.bmin;
-    a.order_pairs = p->b.order_pairs;
-    a.bucket_end = p->b.buckets;
-    a.item_off = p->item_off;
-    a.c_order = idx->c_by_size;
-    a.item_counter = p->counter;
-    a.K = K;
-    a.D = (int)idx->D;
-    a.nprobe = (int)p->nprobe_run;
-    a.CB = (int)t.blocks_per_item;
-    (void)nq;
-    ERQ_TRY(tc_status_ptr(&a.status));
+    ERQ_TRY(scan_work_list(p->idx, p->b, p->nprobe_run, (int)t.queries_per_item, (int)t.blocks_per_item, a, st));
     const int qb = (int)t.queries_per_item, w = (int)t.warps;
     auto grid = [&](int i) { return p->sms * p->per_sm[i]; };
     if (qb == 1 && w == 4) return scan_batched_launch<1, 4>(a, grid(0), st);
@@ -3072,7 +3190,7 @@ erq_status plan_pipeline(erq_plan* p, uint64_t nq, const erq_plan_tuning& t, cud
         ERQ_TRY(launch_probe_tc(idx, b, p->nprobe_run, st));
     }
     ERQ_TRY(order_both(idx, b, p->nprobe_run, st, qnp, false));
-    ERQ_TRY(launch_scan_batched(p, nq, t, st));
+    ERQ_TRY(launch_scan_batched(p, t, st));
     ERQ_TRY(launch_refine(idx, b, p->nprobe_run, p->k, p->ids, p->dists, st, qnp, b.order_q,
                           (int)t.refine_warps));
     return ERQ_OK;
@@ -3240,15 +3358,14 @@ erq_status erq_plan_create(const erq_index* idx, const erq_probe_model* model, u
         ERQ_TRY((scan_batched_configure<4, 4>(D, &p->per_sm[4])));
         ERQ_TRY((scan_batched_configure<4, 8>(D, &p->per_sm[5])));
     }
-    ERQ_TRY(alloc_batch(p->arena, idx, max_batch, p->nprobe_run, p->b));
+    ERQ_TRY(alloc_batch(p->arena, idx, max_batch, p->nprobe_run, p->b,
+                        model ? max_batch : max_batch * p->nprobe_run));
     if (model) ERQ_TRY(alloc_probe_lists(p->arena, max_batch, p->b));
     ERQ_TRY(p->arena.alloc(&p->qin, max_batch * (p->raw ? idx->DIM : idx->D)));
     ERQ_TRY(p->arena.alloc(&p->qrot, max_batch * idx->D));
     ERQ_TRY(p->arena.alloc(&p->ids, max_batch * k));
     ERQ_TRY(p->arena.alloc(&p->dists, max_batch * k));
     ERQ_TRY(p->arena.alloc(&p->used, max_batch));
-    ERQ_TRY(p->arena.alloc(&p->item_off, idx->K + 1));
-    ERQ_TRY(p->arena.alloc(&p->counter, 1));
     if (model) {
         ERQ_TRY(p->arena.alloc(&p->near_d, max_batch * kFeatDists));
         ERQ_TRY(p->arena.alloc(&p->feats, max_batch * kMlpIn));
@@ -3333,6 +3450,7 @@ erq_status erq_plan_autotune(erq_plan* p, const float* queries, uint64_t n, int 
     for (int si = 0; si < kNumScanShapes && s == ERQ_OK; ++si) {
         const ScanShape& sh = kScanShapes[si];
         if (!p->per_sm[si]) continue;  // does not fit at this D
+        if (plan_scans_mma(p, n)) break;  // the tile shapes are the lookup scan's
         for (int cb : kChunkChoices) {
             erq_plan_tuning t = default_tuning(n);  // refinement form by batch size
             t.queries_per_item = (uint32_t)sh.qb;
