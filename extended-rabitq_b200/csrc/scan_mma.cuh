@@ -242,7 +242,8 @@ __global__ void __launch_bounds__(kMmaThreads, 2)
 scan_mma_kernel(const __grid_constant__ CUtensorMap rows, uint32_t cap, ScanBatchArgs a) {
     extern __shared__ uint8_t smem_raw[];
     const int D = a.D;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // known uniform to the compiler
     const uint32_t raw = (uint32_t)__cvta_generic_to_shared(smem_raw);
     const uint32_t bop = (raw + 1023u) & ~1023u;  // B operand
     uint64_t* bars_p = reinterpret_cast<uint64_t*>(smem_raw + (bop - raw) + mma_b_bytes(D));
