@@ -497,11 +497,6 @@ erq_status load_impl(const char* path, erq_index* idx) {
 }
 
 // ------------------------------------------------------------ pipeline
-size_t refine_smem_bytes(int D, int k, bool wide = false) {
-    const int kpad = (k + 31) & ~31;
-    return refine_smem_bytes_per_query(D, kpad, wide ? kWideWindowBlocks : kWindowBlocks);
-}
-
 // Streaming multiprocessors of the current device (cached per device).
 int device_sms() {
     static int sms[64] = {};
@@ -516,18 +511,19 @@ int device_sms() {
     return sms[dev];
 }
 
-// The limits cover the largest k, so a later call with a smaller k never
-// lowers them below what a captured graph's launches need.
+// The limit covers every D and k, so a call never lowers it below what a
+// captured graph's launches need.
 template <int EX>
-erq_status configure_refine(int D) {
-    ERQ_CUDA(cudaFuncSetAttribute(refine_kernel<EX, 4, kWindowBlocks>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)refine_smem_bytes(D, kMaxTopK)));
-    ERQ_CUDA(cudaFuncSetAttribute(refine_kernel<EX, kWideWarps, kWideWindowBlocks>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)refine_smem_bytes(D, kMaxTopK, true)));
+erq_status configure_refine() {
+    ERQ_CUDA(cudaFuncSetAttribute(refine_kernel<EX, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
+    ERQ_CUDA(cudaFuncSetAttribute(refine_kernel<EX, kWideWarps>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  220 * 1024));
     return ERQ_OK;
 }
+static_assert(refine_smem_bytes<4>(kMaxD, kMaxTopK) <= 64 * 1024 &&
+                  refine_smem_bytes<kWideWarps>(kMaxD, kMaxTopK) <= 220 * 1024 &&
+                  refine_smem_bytes<kWideWarps>(kMaxD, 32) <= 220 * 1024,
+              "shared memory of the refinement");
 int next_pow2(int x) {
     int p = 1;
     while (p < x) p <<= 1;
@@ -559,12 +555,12 @@ erq_status configure_kernels(int D, int K, int k) {
         ERQ_CUDA(cudaFuncSetAttribute(refine_lowacc_kernel<7>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
         ERQ_CUDA(cudaFuncSetAttribute(refine_lowacc_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     }
-    ERQ_TRY(configure_refine<2>(D));
-    ERQ_TRY(configure_refine<3>(D));
-    ERQ_TRY(configure_refine<4>(D));
-    ERQ_TRY(configure_refine<6>(D));
-    ERQ_TRY(configure_refine<7>(D));
-    ERQ_TRY(configure_refine<8>(D));
+    ERQ_TRY(configure_refine<2>());
+    ERQ_TRY(configure_refine<3>());
+    ERQ_TRY(configure_refine<4>());
+    ERQ_TRY(configure_refine<6>());
+    ERQ_TRY(configure_refine<7>());
+    ERQ_TRY(configure_refine<8>());
     return ERQ_OK;
 }
 
@@ -1265,7 +1261,7 @@ erq_status launch_scan_mma(const erq_index* idx, const Batch& b, uint64_t nprobe
     return ERQ_OK;
 }
 
-// refine_warps: 4 or kWideWarps chooses the form; 0 takes the wide one when
+// refine_warps: 4 or kWideTuning chooses the form; 0 takes the wide one when
 // the batch has no more queries than SMs.
 erq_status launch_refine(const erq_index* idx, const Batch& b, uint64_t nprobe, uint64_t k,
                          uint32_t* out_ids, float* out_dists, cudaStream_t st,
@@ -1345,15 +1341,16 @@ erq_status launch_refine(const erq_index* idx, const Batch& b, uint64_t nprobe, 
     a.nprobe = (int)nprobe;
     a.k = (int)k;
     const unsigned grid = (unsigned)b.nq;
-    const bool wide = refine_warps ? refine_warps == kWideWarps : b.nq <= (uint64_t)device_sms();
-    const size_t smem = refine_smem_bytes(a.D, a.k, wide);
+    const bool wide = refine_warps ? refine_warps == kWideTuning : b.nq <= (uint64_t)device_sms();
+    const int kpad = (a.k + 31) & ~31;
+    const size_t smem = wide ? refine_smem_bytes<kWideWarps>(a.D, kpad) : refine_smem_bytes<4>(a.D, kpad);
     LaunchTimer t(kRefine, st);
 #define ERQ_REFINE_CASE(X)                                                                          \
     case X:                                                                                         \
         if (wide)                                                                                   \
-            refine_kernel<X, kWideWarps, kWideWindowBlocks><<<grid, kWideWarps * 32, smem, st>>>(a); \
+            refine_kernel<X, kWideWarps><<<grid, kWideWarps * 32, smem, st>>>(a); \
         else                                                                                        \
-            refine_kernel<X, 4, kWindowBlocks><<<grid, kRefineThreads, smem, st>>>(a);              \
+            refine_kernel<X, 4><<<grid, kRefineThreads, smem, st>>>(a);              \
         break;
     switch (idx->EX) {
         ERQ_REFINE_CASE(2)
@@ -3133,7 +3130,7 @@ bool tuning_valid(const erq_plan_tuning& t) {
     bool shape = false;
     for (auto& sh : kScanShapes) shape |= (int)t.queries_per_item == sh.qb && (int)t.warps == sh.warps;
     return shape && t.blocks_per_item >= 1 && t.blocks_per_item <= 4096 &&
-           (t.refine_warps == 0 || t.refine_warps == 4 || t.refine_warps == (uint32_t)kWideWarps);
+           (t.refine_warps == 0 || t.refine_warps == 4 || t.refine_warps == (uint32_t)kWideTuning);
 }
 
 // Whether the plan's batches of nq queries scan on the tensor cores (a learned
@@ -3476,7 +3473,7 @@ erq_status erq_plan_autotune(erq_plan* p, const float* queries, uint64_t n, int 
         if (s != ERQ_OK) break;
     }
     // both refinement forms with the chosen tile (the auto choice is one of them)
-    for (uint32_t rw : {4u, (uint32_t)kWideWarps}) {
+    for (uint32_t rw : {4u, (uint32_t)kWideTuning}) {
         if (s != ERQ_OK) break;
         erq_plan_tuning t = bt;
         t.refine_warps = rw;
@@ -3496,7 +3493,7 @@ erq_status erq_plan_autotune(erq_plan* p, const float* queries, uint64_t n, int 
             bt = t;
         }
     }
-    if (bt.refine_warps == 0) bt.refine_warps = n <= (uint64_t)device_sms() ? kWideWarps : 4;
+    if (bt.refine_warps == 0) bt.refine_warps = n <= (uint64_t)device_sms() ? kWideTuning : 4;
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     ERQ_TRY(s);

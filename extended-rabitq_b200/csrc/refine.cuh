@@ -1,12 +1,12 @@
 // Lower-bound test, EX-bit refinement and the per-query top-k pool.
 //
-// One warp per query replays the reference's sequential scan order
+// One block per query replays the reference's sequential scan order
 // (inc/index/IVF.hpp:313-321, inc/index/HASearcher.hpp:82-112,187-236):
 // clusters in probe order, blocks in storage order, candidates of a block in
 // ascending lane order.  The block's candidate mask is taken against the
 // top-k threshold as it stands when the block starts; every candidate is
 // offered to the pool in order and the threshold is refreshed after each
-// insertion.  The integer sums S come from the scan kernel; everything that
+// insertion.  The integer sums S come from the scan kernels; everything that
 // depends on the threshold happens here, so the candidate sets and the
 // returned ids and distances equal the reference's.
 //
@@ -54,8 +54,15 @@ struct RefineArgs {
 };
 
 
-// Codes of bytes (lo, lo+1) of w as exact floats: 0x4B0000vv is 2^23 + v.
+// Codes of bytes (lo, lo+1) of w as floats.  SCALED: the byte v in bits 16-23
+// of a float is exactly v * 2^-133 (subnormal below 128, and the exponent's
+// lowest bit carries on the same spacing above): one instruction per code.
+// Otherwise exact integers: 0x4B0000vv is 2^23 + v.
+template <bool SCALED>
 __device__ __forceinline__ float2 code_pair(uint32_t w, int lo) {
+    if (SCALED)
+        return make_float2(__int_as_float((int)__byte_perm(w, 0u, 0x4044u | ((uint32_t)lo << 8))),
+                           __int_as_float((int)__byte_perm(w, 0u, 0x4044u | ((uint32_t)(lo + 1) << 8))));
     const float2 big = make_float2(__int_as_float((int)__byte_perm(w, 0x4B000000u, 0x7540u | (uint32_t)lo)),
                                    __int_as_float((int)__byte_perm(w, 0x4B000000u, 0x7540u | (uint32_t)(lo + 1))));
     return fsub2(big, make_float2(8388608.f, 8388608.f));
@@ -72,9 +79,22 @@ __device__ __forceinline__ uint32_t step_word(const uint4& v, int t) {
 
 // One step of one candidate: accumulators 4r+0..4r+3 of the reference's 16
 // (as two pairs) take fma(unit_q[16s + 4r + i], code, acc).
+template <bool SCALED>
 __device__ __forceinline__ void ip_step(float2 acc[2], const float4& u, uint32_t w) {
-    acc[0] = ffma2(make_float2(u.x, u.y), code_pair(w, 0), acc[0]);
-    acc[1] = ffma2(make_float2(u.z, u.w), code_pair(w, 2), acc[1]);
+    acc[0] = ffma2(make_float2(u.x, u.y), code_pair<SCALED>(w, 0), acc[0]);
+    acc[1] = ffma2(make_float2(u.z, u.w), code_pair<SCALED>(w, 2), acc[1]);
+}
+
+// The reduce tree over a quad's 16 accumulators: acc[l] + acc[l+8], then + 4,
+// then (0 + 2) + (1 + 3); the sum in every lane of the quad.
+__device__ __forceinline__ float ip_tree(const float2 acc[2]) {
+    float t3[4], t6[4];
+    const float a4[4] = {acc[0].x, acc[0].y, acc[1].x, acc[1].y};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) t3[i] = __fadd_rn(__shfl_xor_sync(0xffffffffu, a4[i], 2), a4[i]);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) t6[i] = __fadd_rn(__shfl_xor_sync(0xffffffffu, t3[i], 1), t3[i]);
+    return __fadd_rn(__fadd_rn(t6[0], t6[2]), __fadd_rn(t6[1], t6[3]));
 }
 
 // <unit_q, ex code> of NC (1 or 2) candidates by the 4 lanes r = 0..3 of a
@@ -82,9 +102,8 @@ __device__ __forceinline__ void ip_step(float2 acc[2], const float4& u, uint32_t
 // accumulators acc[l] take the dims l, l+16, l+32, ... in turn; lane r holds
 // acc[4r..4r+3].  Rows are in the lane-interleaved layout of layout.cuh;
 // each lane streams its own uint4s one ahead (a loop unrolled by 3, then the
-// last pass, which fetches nothing).  uq4 = unit_q as float4.
-// Returns the sums (the reduce tree: acc[l] + acc[l+8], then + 4, then
-// (0 + 2) + (1 + 3)) in every lane of the quad.
+// last pass, which fetches nothing).  uq4 = unit_q as float4.  Returns the
+// sums in every lane of the quad.
 template <int SB, int NC>
 __device__ __forceinline__ void ex_ip_quad(const float4* __restrict__ uq4, const uint4* __restrict__ row0,
                                            const uint4* __restrict__ row1, int r, int steps,
@@ -118,7 +137,7 @@ __device__ __forceinline__ void ex_ip_quad(const float4* __restrict__ uq4, const
         for (int t = 0; t < SPU; ++t) {
             const float4 q = qp[4 * t];
 #pragma unroll
-            for (int c = 0; c < NC; ++c) ip_step(acc[c], q, step_word<SB>(cur[c], t));
+            for (int c = 0; c < NC; ++c) ip_step<false>(acc[c], q, step_word<SB>(cur[c], t));
         }
         qp += 4 * SPU;
 #pragma unroll
@@ -129,38 +148,176 @@ __device__ __forceinline__ void ex_ip_quad(const float4* __restrict__ uq4, const
         for (int t = 0; t < SPU; ++t) {
             const float4 q = qp[4 * t];
 #pragma unroll
-            for (int c = 0; c < NC; ++c) ip_step(acc[c], q, step_word<SB>(cur[c], t));
+            for (int c = 0; c < NC; ++c) ip_step<false>(acc[c], q, step_word<SB>(cur[c], t));
         }
         qp += 4 * SPU;
     }
     for (int t = 0; t < steps - Uf * SPU; ++t) {  // a partly filled last uint4
         const float4 q = qp[4 * t];
 #pragma unroll
-        for (int c = 0; c < NC; ++c) ip_step(acc[c], q, step_word<SB>(cur[c], t));
+        for (int c = 0; c < NC; ++c) ip_step<false>(acc[c], q, step_word<SB>(cur[c], t));
     }
 #pragma unroll
-    for (int c = 0; c < NC; ++c) {
-        float t3[4], t6[4];
-        const float a4[4] = {acc[c][0].x, acc[c][0].y, acc[c][1].x, acc[c][1].y};
+    for (int c = 0; c < NC; ++c) out[c] = ip_tree(acc[c]);
+}
+
+// The same for two candidates (or one) of a quad whose rows come through a
+// ring of kRowRing stages of asynchronous 16-byte copies, every lane copying
+// and reading its own words: with one register-fed row word in flight per lane
+// a pass waited for L2 (about 700 cycles for 16 codes a lane).  U: uint4s per
+// lane of a row; uq4 = unit_q * 2^127, zero past D up to U whole uint4s, so
+// every sum is the plain one times 2^-6; ring: this lane's 16 bytes of stage 0,
+// candidate 0 (stages 1024 bytes apart, candidates 512).
+constexpr int kRowRing = 4;
+__device__ __forceinline__ void row_copy(uint32_t dst, const uint4* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void row_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int SB, int NC>
+__device__ __forceinline__ void ex_ip_ring(const float4* __restrict__ uq4, const uint4* __restrict__ row0,
+                                           const uint4* __restrict__ row1, int r, int U, uint32_t ring,
+                                           float out[2]) {
+    constexpr int SPU = 32 / SB;  // steps per uint4
+    float2 acc[NC][2];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) t3[i] = __fadd_rn(__shfl_xor_sync(0xffffffffu, a4[i], 2), a4[i]);
+    for (int c = 0; c < NC; ++c) acc[c][0] = acc[c][1] = make_float2(0.f, 0.f);
+    const uint4* rp[NC];
+    rp[0] = row0 + r;
+    if (NC > 1) rp[NC - 1] = row1 + r;
+    const float4* qp = uq4 + r;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) t6[i] = __fadd_rn(__shfl_xor_sync(0xffffffffu, t3[i], 1), t3[i]);
-        out[c] = __fadd_rn(__fadd_rn(t6[0], t6[2]), __fadd_rn(t6[1], t6[3]));
+    for (int s = 0; s < kRowRing - 1; ++s) {
+        if (s < U) {
+#pragma unroll
+            for (int c = 0; c < NC; ++c) row_copy(ring + s * 1024 + c * 512, rp[c] + 4 * s);
+        }
+        row_commit();
     }
+    const auto next_words = [&](int u, uint4 (&cur)[NC]) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(kRowRing - 2) : "memory");
+#pragma unroll
+        for (int c = 0; c < NC; ++c) cur[c] = lds128(ring + (u % kRowRing) * 1024 + c * 512);
+        if (u + kRowRing - 1 < U) {
+#pragma unroll
+            for (int c = 0; c < NC; ++c)
+                row_copy(ring + ((u + kRowRing - 1) % kRowRing) * 1024 + c * 512, rp[c] + 4 * (u + kRowRing - 1));
+        }
+        row_commit();
+    };
+#pragma unroll 4
+    for (int u = 0; u < U; ++u) {
+        uint4 cur[NC];
+        next_words(u, cur);
+#pragma unroll
+        for (int t = 0; t < SPU; ++t) {
+            const float4 q = qp[4 * t];
+#pragma unroll
+            for (int c = 0; c < NC; ++c) ip_step<true>(acc[c], q, step_word<SB>(cur[c], t));
+        }
+        qp += 4 * SPU;
+    }
+#pragma unroll
+    for (int c = 0; c < NC; ++c) out[c] = __fmul_rn(ip_tree(acc[c]), 64.f);  // the scale: exact
+}
+
+// One candidate with the plain codes (kUnitScale below), a step at a time.
+template <int SB>
+__device__ __forceinline__ float ex_ip_plain(const float4* __restrict__ uq4, const uint4* __restrict__ row, int r,
+                                             int steps) {
+    constexpr int SPW = 8 / SB;  // steps per 32-bit word
+    const uint32_t* words = reinterpret_cast<const uint32_t*>(row + r);
+    float2 acc[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+#pragma unroll 1
+    for (int t = 0; t < steps; ++t) {
+        const int j = t / SPW;  // word j of this lane: word j % 4 of its uint4 j / 4
+        const uint32_t w = __ldg(words + 16 * (j >> 2) + (j & 3)) >> (SB * (t % SPW));
+        ip_step<false>(acc, uq4[4 * t + r], SB == 8 ? w : w & (0x01010101u * ((1u << SB) - 1u)));
+    }
+    return ip_tree(acc);
+}
+
+// unit_q is staged times 2^127 for the scaled codes.  With every non-zero
+// |unit_q| in [2^-96, 2) the products and sums are multiples of 2^-125 below
+// 2^128 in the scaled form, so each rounding is that of the plain one; a
+// cluster whose unit query leaves that range (never, for data of ordinary
+// magnitudes: its norm is 1) takes the plain codes.
+constexpr float kUnitScale = 1.7014118346046923e38f;  // 2^127
+__device__ __forceinline__ bool unit_scales(float u) {
+    const float a = fabsf(u);
+    return a == 0.f || (a >= 1.262177448e-29f && a < 2.f);  // 2^-96; false for NaN
 }
 
 constexpr int kRefineThreads = 128;     // 4 warps per query
-constexpr int kWindowBlocks = 16;       // blocks whose candidates are refined together
-constexpr int kFirstWindowBlocks = 8;   // the same in the query's first probed cluster
-// Wide form for small batches (a query per SM): more warps, longer windows.
-constexpr int kWideWarps = 32;
-constexpr int kWideWindowBlocks = 128;
+// Wide form for small batches (a query per SM): more warps, longer lists.
+constexpr int kWideWarps = 16;
+constexpr int kWideTuning = 32;  // erq_plan_tuning's refine_warps of the wide form
 
-// Shared memory of one block: unit_q[D] | per window lane: lb, ipq, onorm,
-// ex_dist, id, list | pool_d[kpad] | pool_id[kpad] | misc | window blocks
-__host__ __device__ constexpr size_t refine_smem_bytes_per_query(int D, int kpad, int wb) {
-    return (size_t)D * 4 + (size_t)wb * 32 * (5 * 4 + 2) + (size_t)kpad * 8 + 64 + 128 + (size_t)wb * 4;
+// Window capacities of the two forms: listed candidates, clusters whose unit
+// queries are staged at once (at most), block minima tested per thread.
+template <int WARPS>
+struct RefineForm {
+    static constexpr int kBlocks = WARPS == 4 ? 16 : 32;     // most blocks of a window (a lane each)
+    static constexpr int kEntries = WARPS == 4 ? 256 : 1024;
+    static constexpr int kSlots = WARPS == 4 ? 8 : 16;
+    static constexpr int kPerThread = WARPS == 4 ? 4 : 2;
+    static constexpr int kWords = WARPS * kPerThread;  // 32 blocks each
+    static constexpr int kProbes = WARPS == 4 ? 128 : 256;  // probes whose clusters are kept
+    // shared memory of a block: 6 blocks of the 4-warp form per SM (1,284 us of
+    // learned refinement with 5, 1,191 with 6; with 8 the ring does not fit,
+    // 1,233), one of the wide form
+    static constexpr int kRoom = WARPS == 4 ? 36 * 1024 + 512 : 220 * 1024;
+    static constexpr int kPerSm = WARPS == 4 ? 6 : 1;
+};
+
+template <int WARPS>
+struct RefineShared {
+    using F = RefineForm<WARPS>;
+    uint4 ring[WARPS][kRowRing][2][32];  // EX-code words (ex_ip_ring)
+    // slots: clusters whose unit queries are staged
+    double ex_sub[F::kSlots];
+    float y[F::kSlots], fac[F::kSlots], sqy[F::kSlots], delta[F::kSlots];
+    uint32_t cid[F::kSlots], plain[F::kSlots];
+    // blocks of the window
+    float4 k[F::kBlocks];           // delta, c1, c2, c3 (LbConsts)
+    uint32_t block[F::kBlocks];     // among the query's blocks
+    uint32_t probe[F::kBlocks];
+    uint32_t vec[F::kBlocks];       // position of lane 0's vector
+    uint32_t on[F::kBlocks];        // index of its block factor
+    uint32_t cid_of[F::kBlocks];
+    float sqy_of[F::kBlocks], sumq_of[F::kBlocks];
+    uint32_t lanes[F::kBlocks];     // vectors of the block
+    uint32_t mask[F::kBlocks];      // lanes below the threshold
+    uint32_t slot[F::kBlocks];
+    uint32_t words[32];                // block minima below the threshold
+    uint32_t start[F::kProbes], pcid[F::kProbes], psize[F::kProbes];  // first block, cluster, its size
+    // the listed candidates, in scan order; a block's list is padded to an
+    // even length (kNoEntry)
+    float d[F::kEntries];
+    uint32_t id[F::kEntries];
+    uint16_t list[F::kEntries];        // 32 * window block + lane
+    float lb[F::kBlocks * 32];         // lower bounds of the window's lanes
+    float merge[32];                   // scratch of pool_merge_block
+    int got, size;
+    uint32_t next;
+    float distk;
+};
+constexpr uint16_t kNoEntry = 0xffff;
+
+__host__ __device__ constexpr int refine_pool_bytes(int kpad) { return kpad * 8; }  // distance, id
+// Row length of a staged unit query: D up to whole uint4s of 8-, 4- or 2-bit codes.
+__host__ __device__ constexpr int refine_row(int D) { return (D + 255) & ~255; }
+// Unit queries staged at once: what the block's shared memory leaves, at least one.
+template <int WARPS>
+__host__ __device__ constexpr int refine_slots(int D, int kpad) {
+    const int fixed = (int)sizeof(RefineShared<WARPS>) + refine_pool_bytes(kpad);
+    const int room = RefineForm<WARPS>::kRoom - fixed;
+    const int n = room / (4 * refine_row(D));
+    return n < 1 ? 1 : (n > RefineForm<WARPS>::kSlots ? RefineForm<WARPS>::kSlots : n);
+}
+// [RefineShared][pool][unit queries]
+template <int WARPS>
+__host__ __device__ constexpr size_t refine_smem_bytes(int D, int kpad) {
+    return sizeof(RefineShared<WARPS>) + (size_t)refine_pool_bytes(kpad) + (size_t)refine_slots<WARPS>(D, kpad) * refine_row(D) * 4;
 }
 
 // Order key: ascending distance (-0 equal to +0, as float compares see it);
@@ -286,259 +443,591 @@ __device__ __forceinline__ void pool_merge_block(float* pool_d, uint32_t* pool_i
     distk = size == k ? pool_d[k - 1] : FLT_MAX;
 }
 
-// One block of WARPS warps per query (4, or 32 in the wide form).  Per window
-// of up to WB blocks of the current cluster (16, or 128; 8 in a query's first
-// cluster in the 4-warp form): the warps compute the lower bounds of the
-// window's blocks, dealt round robin, and list the lanes below the threshold
-// as it stands at the window's start (a superset of the exact candidates,
-// because the threshold only falls); the quads compute the listed candidates'
-// exact distances (8 quads per warp; warps without a candidate skip the
-// round); warp 0 then replays the window in the reference's order -
-// each block's mask against the threshold at that block's start, the block's
-// candidates merged into the pool as inserting them in lane order would.
-template <int EX, int WARPS, int WB>
-__global__ void __launch_bounds__(WARPS * 32, WARPS == 4 ? 8 : 1) refine_kernel(RefineArgs a) {
-    constexpr int kThreads = WARPS * 32, kLanes = WB * 32;
-    static_assert(WB % WARPS == 0 && kLanes <= 65536, "window lanes are listed as u16");
+// pool_merge_block on a pool whose size and threshold lie in shared memory,
+// out of line: only pools above kSmallPool entries use it.
+__device__ __noinline__ void pool_merge_shared(float* pool_d, uint32_t* pool_id, int* size_s, float* distk_s,
+                                               int k, bool cand, float d, uint32_t id, float* cs, int lane,
+                                               bool count_all) {
+    int size = *size_s;
+    float distk = *distk_s;
+    __syncwarp();
+    pool_merge_block(pool_d, pool_id, size, k, distk, cand, d, id, cs, lane, count_all);
+    if (lane == 0) {
+        *size_s = size;
+        *distk_s = distk;
+    }
+    __syncwarp();
+}
+
+// The query's top-k pool.  ResultPool (inc/index/Pool.hpp:10-50) keeps the k
+// smallest under the order (distance, newer first): a new value goes before
+// equal ones, an equal value still enters a full pool and pushes the last one
+// out, a larger one is rejected.  Up to kSmallPool entries warp 0 keeps a full
+// pool sorted in registers, place p in lane p % 32: the order of the distance
+// and the id, at the top places; those below hold order 0.  An insertion moves
+// the entries not below the new one up a place, the largest out: about 45
+// instructions without a branch (merging each block's candidates into a sorted
+// pool in shared memory took about 600 per block).  Larger pools stay in shared
+// memory (pool_merge_block).
+constexpr int kSmallPool = 256;
+// Order of a distance as an unsigned number (-0 as +0, as float compares see it).
+__device__ __forceinline__ uint32_t float_order(float x) {
+    const uint32_t b = __float_as_uint(x == 0.f ? 0.f : x);
+    return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
+}
+__device__ __forceinline__ float order_float(uint32_t o) {
+    return __uint_as_float((o & 0x80000000u) ? (o & 0x7fffffffu) : ~o);
+}
+struct SmallPool {
+    static constexpr int kRows = kSmallPool / 32;
+    uint32_t v[kRows], id[kRows];  // the first R rows, R = 1, 4 or 8 by k
+
+    // n entries (distance and id in d and ids, entry e the e-th insertion),
+    // sorted by counting.  scratch: 64 * R words.  (A loop over the entries: a
+    // sorting network in registers is 1,400 instructions run once a query.)
+    template <int R>
+    __device__ __forceinline__ void fill(const float* d, const uint32_t* ids, int n, int lane, uint32_t* scratch) {
+        uint32_t* sid = scratch + 32 * R;
+        int at[R];
+#pragma unroll
+        for (int j = 0; j < R; ++j) {
+            const int e = lane + 32 * j;
+            v[j] = e < n ? float_order(d[e]) : 0u;
+            id[j] = e < n ? ids[e] : 0u;
+            at[j] = 32 * R - n;
+            scratch[e] = v[j];
+        }
+        __syncwarp();
+#pragma unroll(R == 8 ? 4 : 8)
+        for (int e = 0; e < n; ++e) {
+            const uint32_t x = scratch[e];
+#pragma unroll
+            for (int j = 0; j < R; ++j)  // of equal ones the newer comes first
+                at[j] += x < v[j] + (uint32_t)(e > lane + 32 * j);
+        }
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < R; ++j) {
+            const int e = lane + 32 * j, to = e < n ? at[j] : e - n;
+            scratch[to] = v[j];
+            sid[to] = id[j];
+        }
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < R; ++j) {
+            v[j] = scratch[lane + 32 * j];
+            id[j] = sid[lane + 32 * j];
+        }
+        __syncwarp();
+    }
+    // Order of the k-th distance (of a full pool).
+    template <int R>
+    __device__ __forceinline__ uint32_t last() const {
+        return __shfl_sync(0xffffffffu, v[R - 1], 31);
+    }
+    // Inserts (x, vid), x the order of its distance: before equal ones, the
+    // largest entry leaves (x itself when it is larger than all).
+    template <int R>
+    __device__ __forceinline__ void insert(uint32_t x, uint32_t vid, int lane) {
+        uint32_t rv[R], ri[R];
+#pragma unroll
+        for (int j = 0; j < R; ++j) {  // the entries one place down (lane 0: one row up)
+            rv[j] = __shfl_sync(0xffffffffu, v[j], (lane + 31) & 31);
+            ri[j] = __shfl_sync(0xffffffffu, id[j], (lane + 31) & 31);
+        }
+#pragma unroll
+        for (int j = 0; j < R; ++j) {
+            const uint32_t dv = lane ? rv[j] : (j ? rv[j > 0 ? j - 1 : 0] : 0u);
+            const uint32_t di = lane ? ri[j] : (j ? ri[j > 0 ? j - 1 : 0] : 0u);
+            const bool stays = v[j] < x, here = dv < x;
+            id[j] = stays ? id[j] : (here ? vid : di);
+            v[j] = stays ? v[j] : (here ? x : dv);
+        }
+    }
+};
+
+// What a warp needs to replay a window (below).
+struct Replay {
+    const uint16_t* list;
+    const float* d;
+    const float* lb;
+    const uint32_t* ids;
+    float* pool_d;      // the entries of a pool that is not full
+    uint32_t* pool_id;
+    uint32_t* scratch;
+    int entries, k;
+    bool all;           // count every candidate (RefineArgs::stats)
+};
+
+// Replays a window's list in the reference's order: each block's candidates
+// against the threshold at that block's start, those that can enter inserted
+// one by one.  worst: order of the threshold, order of FLT_MAX while the pool
+// fills.
+template <int R>
+__device__ __forceinline__ void replay_window(const Replay& w, SmallPool& sp, int& size, uint32_t& worst,
+                                              uint32_t& st_cand, int lane) {
+    const uint32_t lt = (1u << lane) - 1u;
+    int cur = -1;  // block the replay is in, and the threshold at its start
+    uint32_t at_start = worst;
+#pragma unroll 1
+    for (int e0 = 0; e0 < w.entries; e0 += 32) {
+        const int e = e0 + lane;
+        const uint32_t l = e < w.entries ? w.list[e] : kNoEntry;
+        const bool valid = l != kNoEntry;
+        const float d = valid ? w.d[e] : 0.f;
+        const uint32_t od = float_order(d), ol = float_order(valid ? w.lb[l] : 0.f);
+        const uint32_t vid = valid ? w.ids[e] : 0u;
+        const int blk = (int)(l >> 5);
+        // those above a full pool's k-th cannot enter
+        uint32_t todo = __ballot_sync(0xffffffffu, valid && (w.all || size < w.k || od <= worst));
+        if (size < w.k && todo) {
+            // the pool fills: its blocks started without a threshold, so
+            // every listed lane is a candidate
+            const int at = size + __popc(todo & lt);
+            const bool take = ((todo >> lane) & 1u) && at < w.k;
+            if (take) {
+                w.pool_d[at] = d;
+                w.pool_id[at] = vid;
+            }
+            const uint32_t taken = __ballot_sync(0xffffffffu, take);
+            cur = __shfl_sync(0xffffffffu, blk, 31 - __clz((int)taken));
+            size += __popc(taken);
+            if (w.all) st_cand += __popc(taken);
+            todo &= ~taken;
+            __syncwarp();
+            if (size == w.k) {
+                sp.fill<R>(w.pool_d, w.pool_id, w.k, lane, w.scratch);
+                worst = sp.last<R>();
+                todo &= __ballot_sync(0xffffffffu, w.all || od <= worst);
+            }
+        }
+#pragma unroll 1
+        while (todo) {  // a block at a time
+            const int b = __shfl_sync(0xffffffffu, blk, __ffs(todo) - 1);
+            if (b != cur) {
+                cur = b;
+                at_start = sp.last<R>();
+            }
+            const bool mine = ((todo >> lane) & 1u) && blk == b;
+            const bool candidate = mine && ol < at_start;
+            todo &= ~__ballot_sync(0xffffffffu, mine);
+            if (w.all) st_cand += __popc(__ballot_sync(0xffffffffu, candidate));
+            // a larger distance than the largest leaves the pool as it is
+            uint32_t in = __ballot_sync(0xffffffffu, candidate && od <= at_start);
+#pragma unroll 1
+            while (in) {
+                const int src = __ffs(in) - 1;
+                in &= in - 1u;
+                sp.insert<R>(__shfl_sync(0xffffffffu, od, src), __shfl_sync(0xffffffffu, vid, src), lane);
+            }
+        }
+        if (size == w.k) worst = sp.last<R>();
+    }
+}
+
+// The sorted pool to the query's results.
+template <int R>
+__device__ __forceinline__ void pool_out(SmallPool& sp, const Replay& w, int size, uint32_t* oid, float* od,
+                                         int lane) {
+    if (size < w.k) sp.fill<R>(w.pool_d, w.pool_id, size, lane, w.scratch);
+#pragma unroll
+    for (int j = 0; j < R; ++j) {
+        const int i = lane + 32 * j - (32 * R - size);
+        if (i >= 0) {
+            oid[i] = sp.id[j];
+            if (od) od[i] = order_float(sp.v[j]);
+        }
+    }
+}
+
+// One block of WARPS warps per query (4, or 16 in the wide form).  The query's
+// blocks - of all its probed clusters, in probe order - form one sequence; a
+// window is the next of them whose smallest lower bound (from the scan) is
+// below the threshold at the window's start (a block above it has no candidate
+// then or later), whatever clusters they belong to.  The warps compute the
+// lower bounds of the window's blocks and list the lanes below the threshold -
+// a superset of the exact candidates, because the threshold only falls; the
+// quads compute the listed candidates' exact distances against the staged unit
+// queries; warp 0 then replays the window in the reference's order: each
+// block's candidates against the threshold at that block's start, those that
+// can enter inserted one by one.
+// A window ends early when its list is full, when its candidates come from
+// more clusters than unit queries fit, or, while the pool fills (every lane is
+// a candidate), once it can fill it; its length never changes a result.
+// Windows across clusters keep the quads busy where a cluster has a few
+// candidates: with a window per cluster (and up to 16 of its blocks) 2,047
+// queries at nprobe 96 over Zipf clusters took 109 windows each and 5.41 ms, now
+// 40 and 4.45 ms; 64 queries at nprobe 128 129 and 1.12 ms, now 14 and 0.56 ms;
+// 2,000 queries at nprobe 64 over even clusters 67 and 1.47 ms, now 4 and 0.92 ms;
+// one query of 128 dims at nprobe 32 88 us, now 35 us.
+template <int EX, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32, RefineForm<WARPS>::kPerSm) refine_kernel(RefineArgs a) {
+    using F = RefineForm<WARPS>;
+    constexpr int kThreads = WARPS * 32;
+    constexpr int kOwn = F::kBlocks / WARPS;  // window blocks per warp
+    constexpr int SB = ex_storage_bits(EX);
     extern __shared__ __align__(16) uint8_t smem_raw[];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    RefineShared<WARPS>& sh = *reinterpret_cast<RefineShared<WARPS>*>(smem_raw);
+    const int tid = threadIdx.x, lane = tid & 31;
+    // through a shuffle, so that the compiler knows it uniform over the warp and
+    // the warp-wide operations of the branches on it need no resynchronisation
+    const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+    const uint32_t lt = (1u << lane) - 1u;
     const int q = a.order ? (int)a.order[blockIdx.x] : (int)blockIdx.x;
-    const int D = a.D, k = a.k;
-    const int kpad = (k + 31) & ~31;
-    float* uq = reinterpret_cast<float*>(smem_raw);
-    float* w_lb = uq + D;
-    float* w_ipq = w_lb + kLanes;
-    float* w_on = w_ipq + kLanes;
-    float* w_ed = w_on + kLanes;
-    uint32_t* w_id = reinterpret_cast<uint32_t*>(w_ed + kLanes);
-    uint16_t* w_list = reinterpret_cast<uint16_t*>(w_id + kLanes);
-    float* pool_d = reinterpret_cast<float*>(w_list + kLanes);
+    const int D = a.D, k = a.k, kpad = (k + 31) & ~31;
+    const int nslots = refine_slots<WARPS>(D, kpad), row_len = refine_row(D);
+    const int row_words = (int)ex_row_uint4(D, EX);
+    float* pool_d = reinterpret_cast<float*>(smem_raw + sizeof(RefineShared<WARPS>));
     uint32_t* pool_id = reinterpret_cast<uint32_t*>(pool_d + kpad);
-    int* misc = reinterpret_cast<int*>(pool_id + kpad);  // [0] list count [1] pool size
-    float* s_distk = reinterpret_cast<float*>(misc + 2);
-    float* cs = reinterpret_cast<float*>(misc + 16);  // 32 floats of merge scratch
-    uint32_t* w_blk = reinterpret_cast<uint32_t*>(cs + 32);  // the window's blocks
-    const int fac_rescale = 1 << EX;
+    float* uq = reinterpret_cast<float*>(pool_id + kpad);
+    const uint32_t ring = (uint32_t)__cvta_generic_to_shared(&sh.ring[warp][0][0][lane]);
+    // warp 0's ring is free while it replays
+    Replay rp{sh.list, sh.d, sh.lb, sh.id, pool_d, pool_id, reinterpret_cast<uint32_t*>(&sh.ring[0][0][0][0]), 0, k,
+              a.stats != nullptr};
+    SmallPool sp;            // with size and distk, maintained by warp 0
+    int size = 0;
+    uint32_t worst = float_order(FLT_MAX);  // order of the threshold
     const float one_over_sqrtD = recip_via_double(__fsqrt_rn((float)D));
     const float* qv = a.qrot + (size_t)q * D;
-
-    for (int i = tid; i < kpad; i += blockDim.x) {
-        pool_d[i] = 0.f;
-        pool_id[i] = 0u;
+    const size_t q0 = (size_t)q * a.nprobe;
+    const int np_q = a.q_nprobe ? a.q_nprobe[q] : a.nprobe;
+    const uint64_t s_base = a.s_off[q0];
+    const int32_t* S = a.S + s_base;
+    const float* bmin = a.bmin ? a.bmin + s_base / 32 : nullptr;
+    const auto start_of = [&](int p) -> uint32_t {
+        return p < F::kProbes ? sh.start[p] : (uint32_t)((a.s_off[q0 + p] - s_base) >> 5);
+    };
+    const auto cid_of = [&](int p) -> uint32_t { return p < F::kProbes ? sh.pcid[p] : a.probe_cid[q0 + p]; };
+    const auto size_of = [&](int p) -> uint32_t { return p < F::kProbes ? sh.psize[p] : a.c_size[cid_of(p)]; };
+#pragma unroll 1
+    for (int p = tid; p < np_q && p < F::kProbes; p += kThreads) {
+        const uint32_t c = a.probe_cid[q0 + p];
+        sh.pcid[p] = c;
+        sh.start[p] = (uint32_t)((a.s_off[q0 + p] - s_base) >> 5);
+        sh.psize[p] = a.c_size[c];
     }
     if (tid == 0) {
-        *s_distk = FLT_MAX;
-        misc[1] = 0;  // pool size as seen by all warps
+        sh.distk = FLT_MAX;
+        sh.size = 0;
     }
-    int size = 0;         // pool state, maintained by warp 0
-    float distk = FLT_MAX;
     uint32_t st_cand = 0, st_refined = 0, st_windows = 0, st_blocks = 0;  // with a.stats
+    uint32_t held_probe = 0xffffffffu;  // the last staged cluster's probe, and its slot
+    int held_slot = 0;
     __syncthreads();
+    const uint32_t first_size = sh.psize[0];
+    const uint32_t total = start_of(np_q - 1) + ((size_of(np_q - 1) + 31u) >> 5);
 
-    const int np_q = a.q_nprobe ? a.q_nprobe[q] : a.nprobe;
-    for (int p = 0; p < np_q; ++p) {
-        const size_t qp = (size_t)q * a.nprobe + p;
-        const uint32_t cid = a.probe_cid[qp];
-        const float sqy = a.probe_sqy[qp];
-        const float y = __fsqrt_rn(sqy);
-        const float delta = a.qp_delta[qp];
-        const float sumq = a.qp_sumq[qp];
-        // lower-bound constants (inc/index/fastscan/FastScan.hpp:297-303)
-        const LbConsts lbk = lb_consts(sumq, y, one_over_sqrtD);
-        const double ex_sub = __dmul_rn((double)fac_rescale - 0.5, (double)sumq);
-        const uint32_t n = a.c_size[cid];
-        const uint32_t fb = a.c_first_block[cid];
-        const uint32_t first_vec = a.c_first_vec[cid];
-        const int32_t* S = a.S + a.s_off[qp];
-        const float* bmin = a.bmin ? a.bmin + a.s_off[qp] / 32 : nullptr;
-        const uint32_t nblocks = (n + 31) >> 5;
-        bool uq_ready = false;
-        // The first cluster's threshold falls fast (the pool fills, then
-        // tightens), so a long window there lists many lanes that its replay
-        // drops; later clusters' thresholds barely move and long windows save
-        // barriers.
-        const int wcap = (WARPS == 4 && p == 0) ? kFirstWindowBlocks : WB;
-        for (uint32_t wb = 0; wb < nblocks;) {
-            const float d0 = *s_distk;
-            const int filled = misc[1];
-            // While the pool is filling every lane is a candidate: take just
-            // enough blocks to fill it, so few lanes are refined in vain.
-            const int want = filled < k ? min(wcap, max(1, (k - filled + 31) / 32))
-                                        : wcap;
-            __syncthreads();
-            // warp 0 picks the window: the next `want` blocks from wb whose
-            // smallest lower bound is below the threshold (a block above it
-            // has no candidate now or later: the threshold only falls)
-            if (warp == 0) {
-                int got = 0;
-                uint32_t pos = wb, next = nblocks;
-                while (got < want && pos < nblocks) {
-                    const uint32_t bb = pos + lane;
-                    const bool take = bb < nblocks && (!bmin || bmin[bb] < d0);
-                    const uint32_t m = __ballot_sync(0xffffffffu, take);
-                    const int rank = __popc(m & ((1u << lane) - 1u));
-                    if (take && got + rank < want) w_blk[got + rank] = bb;
-                    const int nm = __popc(m);
-                    if (got + nm >= want) {
-                        // the want-th taken block ends the window
-                        const uint32_t endm = __ballot_sync(0xffffffffu, take && rank == want - got - 1);
-                        next = pos + (uint32_t)(__ffs(endm) - 1) + 1;
-                        got = want;
-                        break;
-                    }
-                    got += nm;
-                    pos += 32;
-                }
-                if (lane == 0) {
-                    misc[0] = 0;
-                    misc[5] = got;
-                    misc[6] = (int)next;
-                }
-            }
-            __syncthreads();
-            const int nbw = misc[5];
-            const uint32_t wnext = (uint32_t)misc[6];
-            // lower bounds and the candidate superset, 4 blocks per warp
+    for (uint32_t pos = 0; pos < total;) {
+        const float d0 = sh.distk;
+        const int need = k - sh.size;  // entries the pool lacks
+        // the next blocks' minima against the threshold
+        const bool open = !bmin || d0 == FLT_MAX;
 #pragma unroll
-            for (int i = 0; i < WB / (kThreads / 32); ++i) {
-                const int b = i * (kThreads / 32) + warp;  // round robin: short windows use every warp
-                if (b < nbw) {  // uniform per warp
-                    const uint32_t blk = w_blk[b];
-                    const float ipq = __fmul_rn(__int2float_rn(S[32 * blk + lane]), delta);
-                    const float on = a.onorm[(size_t)(fb + blk) * 32 + lane];
-                    const float t = lower_bound(ipq, on, lbk);
-                    const bool valid = 32 * blk + lane < n;
-                    // padding lanes never pass (NaN compares false)
-                    w_lb[32 * b + lane] = valid ? t : __int_as_float(0x7fc00000);
-                    w_ipq[32 * b + lane] = ipq;
-                    w_on[32 * b + lane] = on;
-                    const uint32_t m = __ballot_sync(0xffffffffu, valid && t < d0);
-                    int base = 0;
-                    if (lane == 0 && m) base = atomicAdd(&misc[0], __popc(m));
-                    base = __shfl_sync(0xffffffffu, base, 0);
-                    if ((m >> lane) & 1u) {
-                        w_list[base + __popc(m & ((1u << lane) - 1u))] = (uint16_t)(32 * b + lane);
-                        // start the candidate's EX-code row on its way to L2
-                        const size_t pos = (size_t)first_vec + 32 * blk + lane;
-                        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(
-                                         a.excode + pos * a.ex_row),
-                                     "r"((uint32_t)a.ex_row)
-                                     : "memory");
+        for (int i = 0; i < F::kPerThread; ++i) {
+            const uint32_t bb = pos + i * kThreads + tid;
+            // (without a threshold every block may have candidates: no need to look)
+            const uint32_t m = __ballot_sync(0xffffffffu, bb < total && (open || bmin[bb] < d0));
+            if (lane == 0) sh.words[i * WARPS + warp] = m;
+        }
+        __syncthreads();
+        // warp 0 takes the window's blocks and reads what they need, a lane each
+        if (warp == 0) {
+            const int want = need > 0 && first_size >= (uint32_t)k ? min(F::kBlocks, (need + 31) >> 5) : F::kBlocks;
+            uint32_t w = lane < F::kWords ? sh.words[lane] : 0u;
+            int incl = __popc(w);
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += v;
+            }
+            const int all = __shfl_sync(0xffffffffu, incl, 31);
+#pragma unroll 1
+            for (int e = incl - __popc(w); w && e < want; ++e, w &= w - 1u)
+                sh.block[e] = pos + 32 * lane + __ffs(w) - 1;
+            __syncwarp();
+            const int got = min(all, want);
+            if (lane < got) {
+                const uint32_t b = sh.block[lane];
+                int lo = 0, n = np_q;  // the last probe that starts at or before b
+#pragma unroll 1
+                while (n > 1) {
+                    const int h = n >> 1;
+                    if (start_of(lo + h) <= b) {
+                        lo += h;
+                        n -= h;
+                    } else {
+                        n = h;
                     }
                 }
+                const uint32_t cid = cid_of(lo);
+                const float delta = a.qp_delta[q0 + lo], sumq = a.qp_sumq[q0 + lo], sqy = a.probe_sqy[q0 + lo];
+                sh.cid_of[lane] = cid;
+                sh.sqy_of[lane] = sqy;
+                sh.sumq_of[lane] = sumq;
+                // constants of inc/index/fastscan/FastScan.hpp:297-303
+                const LbConsts kc = lb_consts(sumq, __fsqrt_rn(sqy), one_over_sqrtD);
+                const uint32_t r = b - start_of(lo);
+                sh.probe[lane] = (uint32_t)lo;
+                sh.vec[lane] = a.c_first_vec[cid] + 32 * r;
+                sh.on[lane] = (a.c_first_block[cid] + r) * 32;
+                sh.lanes[lane] = min(32u, size_of(lo) - 32 * r);
+                sh.k[lane] = make_float4(delta, kc.c1, kc.c2, kc.c3);
+            }
+            if (lane == 0) {
+                sh.got = got;
+                sh.next = all > want ? sh.block[want - 1] + 1 : min(total, pos + 32u * F::kWords);
+            }
+        }
+        __syncthreads();
+        const int got = sh.got;
+        uint32_t next = sh.next;
+        if (got == 0) {  // uniform
+            pos = next;
+            continue;
+        }
+        // lower bounds, blocks dealt to the warps round robin
+#pragma unroll 4
+        for (int i = 0; i < kOwn; ++i) {
+            const int b = i * WARPS + warp;
+            if (b < got) {  // uniform per warp
+                const float4 kc = sh.k[b];
+                const float on = a.onorm[(size_t)sh.on[b] + lane];
+                const float ipq = __fmul_rn(__int2float_rn(S[32 * (size_t)sh.block[b] + lane]), kc.x);
+                const float lb = lower_bound(ipq, on, LbConsts{kc.y, kc.z, kc.w});
+                const uint32_t m = __ballot_sync(0xffffffffu, lane < (int)sh.lanes[b] && lb < d0);
+                sh.lb[32 * b + lane] = lb;
+                if (lane == 0) sh.mask[b] = m;
+            }
+        }
+        __syncthreads();
+        // every warp: where each block's candidates go, and where the window ends
+        const uint32_t bmask = lane < got ? sh.mask[lane] : 0u;
+        const uint32_t bprobe = lane < got ? sh.probe[lane] : 0u;
+        const int cnt = __popc(bmask), even = (cnt + 1) & ~1;
+        int end = even, seen = cnt;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, end, o), u = __shfl_up_sync(0xffffffffu, seen, o);
+            if (lane >= o) {
+                end += v;
+                seen += u;
+            }
+        }
+        const uint32_t has = __ballot_sync(0xffffffffu, cnt > 0);
+        const int before = 31 - __clz((int)(has & lt));  // the block with candidates before this one
+        const uint32_t pprobe = __shfl_sync(0xffffffffu, bprobe, before & 31);
+        const bool fresh = cnt > 0 && (before < 0 || pprobe != bprobe);
+        const uint32_t freshm = __ballot_sync(0xffffffffu, fresh);
+        const int rank = __popc(freshm & (lt | (1u << lane))) - 1;  // of this block's cluster
+        const bool fits = end <= F::kEntries && rank < nslots && (need <= 0 || seen - cnt < need);
+        const uint32_t out = __ballot_sync(0xffffffffu, !fits && lane < got);
+        const int nb = out ? __ffs(out) - 1 : got;  // blocks of the window, at least one
+        if (nb < got) next = sh.block[nb];
+        const int entries = __shfl_sync(0xffffffffu, end, nb - 1);
+        const uint32_t inm = freshm & (nb < 32 ? (1u << nb) - 1u : 0xffffffffu);
+        const int ns = __popc(inm);  // clusters with candidates
+        // the first one may be staged already, from the window before
+        const uint32_t probe0 = __shfl_sync(0xffffffffu, bprobe, inm ? __ffs(inm) - 1 : 0);
+        const bool held = ns > 0 && probe0 == held_probe;
+        const int slot0 = held ? held_slot : 0;
+        const int slot = rank < 0 ? 0 : (slot0 + rank) % nslots;
+        if (warp == 0 && lane < nb) {
+            sh.slot[lane] = (uint32_t)slot;
+            if (fresh && !(held && rank == 0)) {
+                const float sumq = sh.sumq_of[lane], sqy = sh.sqy_of[lane];
+                sh.cid[slot] = sh.cid_of[lane];
+                sh.plain[slot] = 0u;
+                const float y = __fsqrt_rn(sqy);
+                sh.y[slot] = y;
+                sh.fac[slot] = recip_via_double(y);
+                sh.sqy[slot] = sqy;
+                sh.delta[slot] = sh.k[lane].x;
+                sh.ex_sub[slot] = __dmul_rn((double)(1 << EX) - 0.5, (double)sumq);
+            }
+        }
+        if (ns > 0) {
+            const int lastb = 31 - __clz((int)inm);
+            held_probe = __shfl_sync(0xffffffffu, bprobe, lastb);
+            held_slot = (slot0 + ns - 1) % nslots;
+        }
+#pragma unroll 2
+        for (int i = 0; i < kOwn; ++i) {
+            const int b = i * WARPS + warp;
+            if (b < nb) {
+                const int base = __shfl_sync(0xffffffffu, end - even, b);
+                const uint32_t m = __shfl_sync(0xffffffffu, bmask, b);
+                if ((m >> lane) & 1u) {
+                    const int e = base + __popc(m & lt);
+                    sh.list[e] = (uint16_t)(32 * b + lane);
+                    // start the candidate's EX-code row on its way to L2
+                    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(
+                                     a.excode + ((size_t)sh.vec[b] + lane) * a.ex_row),
+                                 "r"((uint32_t)a.ex_row)
+                                 : "memory");
+                }
+                if (lane == 0 && (__popc(m) & 1)) sh.list[base + __popc(m)] = kNoEntry;
+            }
+        }
+        if (a.stats) {
+            st_refined += __shfl_sync(0xffffffffu, seen, nb - 1);
+            st_windows += 1;
+            st_blocks += nb;
+        }
+        __syncthreads();
+        if (entries == 0) {  // uniform: nothing in this window can pass
+            pos = next;
+            continue;
+        }
+        // unit queries of the clusters not staged yet, scaled; if one of them
+        // leaves the range (never, for ordinary data), all the window's plain
+        bool plain = false;
+        for (bool scaled = true;; scaled = false) {
+            const int r0 = scaled && held ? 1 : 0, g4 = row_len >> 2;
+#pragma unroll 1
+            for (int i = tid; i < (ns - r0) * g4; i += kThreads) {
+                const int r = i / g4, g = i - r * g4, s = (slot0 + r0 + r) % nslots;
+                float4 u = make_float4(0.f, 0.f, 0.f, 0.f);  // past D
+                if (4 * g < D) {
+                    const float fac = sh.fac[s];
+                    if (sh.y[s] > kNormEps) {
+                        const float4 x = reinterpret_cast<const float4*>(qv)[g];
+                        const float4 c = __ldg(reinterpret_cast<const float4*>(a.centroids + (size_t)sh.cid[s] * D) + g);
+                        u = make_float4(__fmul_rn(__fsub_rn(x.x, c.x), fac), __fmul_rn(__fsub_rn(x.y, c.y), fac),
+                                        __fmul_rn(__fsub_rn(x.z, c.z), fac), __fmul_rn(__fsub_rn(x.w, c.w), fac));
+                    } else {  // (float)(1.0 / sqrt(D))
+                        u = make_float4(one_over_sqrtD, one_over_sqrtD, one_over_sqrtD, one_over_sqrtD);
+                    }
+                }
+                if (scaled) {
+                    if (!(unit_scales(u.x) && unit_scales(u.y) && unit_scales(u.z) && unit_scales(u.w)))
+                        sh.plain[s] = 1u;
+                    u = make_float4(__fmul_rn(u.x, kUnitScale), __fmul_rn(u.y, kUnitScale),
+                                    __fmul_rn(u.z, kUnitScale), __fmul_rn(u.w, kUnitScale));
+                }
+                reinterpret_cast<float4*>(uq + (size_t)s * row_len)[g] = u;
             }
             __syncthreads();
-            const int cnt = misc[0];
-            if (a.stats) {
-                st_refined += cnt;
-                st_windows += 1;
-                st_blocks += nbw;
-            }
-            if (cnt == 0) {  // uniform: nothing in this window can pass
-                wb = wnext;
-                continue;
-            }
-            if (!uq_ready) {
-                const float* cv = a.centroids + (size_t)cid * D;
-                if (y > kNormEps) {
-                    const float fac = recip_via_double(y);
-                    for (int i = tid; i < D; i += blockDim.x) uq[i] = __fmul_rn(__fsub_rn(qv[i], cv[i]), fac);
+            if (!scaled) break;
+#pragma unroll 1
+            for (int r = 0; r < ns; ++r) plain |= sh.plain[(slot0 + r) % nslots] != 0u;
+            if (!plain) break;  // uniform
+            held_probe = 0xffffffffu;  // nothing scaled will be left
+            __syncthreads();  // sh.plain is rewritten below for the next window
+        }
+        // exact distances: quad g (lanes 4g..4g+3) takes one candidate while
+        // there are no more than quads, else two of a block; quads past the
+        // end repeat the first so that the warp stays converged
+        {
+            const int g = tid >> 2, r = tid & 3;
+            const bool two = entries > kThreads / 4;
+            const int tasks = two ? entries >> 1 : entries;
+#pragma unroll 1
+            for (int base = 0; base + 8 * warp < tasks; base += kThreads / 4) {
+                const int t = base + g;
+                const int i0 = t < tasks ? (two ? 2 * t : t) : 0;
+                const int s0 = sh.list[i0] == kNoEntry ? sh.list[0] : sh.list[i0];
+                const int i1 = two ? i0 + 1 : i0;
+                const int s1 = two && sh.list[i1] != kNoEntry ? sh.list[i1] : s0;
+                const size_t pos0 = (size_t)sh.vec[s0 >> 5] + (s0 & 31);
+                const size_t pos1 = (size_t)sh.vec[s1 >> 5] + (s1 & 31);
+                const uint4* row0 = reinterpret_cast<const uint4*>(a.excode + pos0 * a.ex_row);
+                const uint4* row1 = reinterpret_cast<const uint4*>(a.excode + pos1 * a.ex_row);
+                // lane 0 of the quad finishes the first, lane 1 the second
+                const int mine = r == 0 ? i0 : i1, sl = r == 0 ? s0 : s1;
+                const int wb = sl >> 5;
+                const bool fin = t < tasks && (r == 0 || (r == 1 && two)) && sh.list[mine] != kNoEntry;
+                const uint32_t cs = sh.slot[wb];
+                float xipn = 0.f, on = 0.f;
+                int sum = 0;
+                uint32_t vid = 0u;
+                if (fin) {
+                    const size_t at = r == 0 ? pos0 : pos1;
+                    xipn = __ldg(a.xipnorm + at);
+                    vid = __ldg(a.ids + at);
+                    on = a.onorm[(size_t)sh.on[wb] + (sl & 31)];
+                    sum = S[32 * (size_t)sh.block[wb] + (sl & 31)];
+                }
+                const float4* uq4 = reinterpret_cast<const float4*>(uq + (size_t)cs * row_len);
+                float ip[2];
+                if (plain) {
+                    ip[0] = ex_ip_plain<SB>(uq4, row0, r, D / 16);
+                    ip[1] = ex_ip_plain<SB>(uq4, row1, r, D / 16);
+                } else if (two) {
+                    ex_ip_ring<SB, 2>(uq4, row0, row1, r, row_words, ring, ip);
                 } else {
-                    const float fill = recip_via_double(__fsqrt_rn((float)D));
-                    for (int i = tid; i < D; i += blockDim.x) uq[i] = fill;
+                    ex_ip_ring<SB, 1>(uq4, row0, row0, r, row_words, ring, ip);
                 }
-                uq_ready = true;
-                __syncthreads();
-            }
-            // refine the listed candidates: quad g (lanes 4g..4g+3) takes two
-            // per round while more than one per quad remain, else one; within a warp
-            // that has work, quads past the end repeat the list's first so
-            // the warp stays converged
-            {
-                const int g = tid >> 2, r = tid & 3;
-                const float4* uq4 = reinterpret_cast<const float4*>(uq);
-                for (int base = 0; base < cnt;) {
-                    const int two = cnt - base > kThreads / 4;
-                    const int step = two ? kThreads / 2 : kThreads / 4;
-                    // per warp: skip when none of its slots holds a candidate,
-                    // one candidate per quad when its second slots are empty
-                    if (base + 8 * warp >= cnt) {
-                        base += step;
-                        continue;
-                    }
-                    const int wtwo = two && base + kThreads / 4 + 8 * warp < cnt;
-                    const int i0 = base + g, i1 = base + kThreads / 4 + g;
-                    const int s0 = w_list[i0 < cnt ? i0 : 0];
-                    const int s1 = w_list[wtwo && i1 < cnt ? i1 : 0];
-                    const size_t pos0 = (size_t)first_vec + 32 * w_blk[s0 >> 5] + (s0 & 31);
-                    const size_t pos1 = (size_t)first_vec + 32 * w_blk[s1 >> 5] + (s1 & 31);
-                    const uint4* row0 = reinterpret_cast<const uint4*>(a.excode + pos0 * a.ex_row);
-                    const uint4* row1 = reinterpret_cast<const uint4*>(a.excode + pos1 * a.ex_row);
-                    // lane 0 of the quad finishes the first, lane 1 the second
-                    const int i = r == 0 ? i0 : i1;
-                    const bool fin = r < 2 && (r == 0 || wtwo) && i < cnt;
-                    const int slot = r == 0 ? s0 : s1;
-                    const size_t pos = r == 0 ? pos0 : pos1;
-                    float xipn = 0.f;
-                    uint32_t vid = 0u;
-                    if (fin) {
-                        xipn = __ldg(a.xipnorm + pos);
-                        vid = __ldg(a.ids + pos);
-                    }
-                    float ip[2];
-                    if (wtwo)
-                        ex_ip_quad<ex_storage_bits(EX), 2>(uq4, row0, row1, r, D / 16, ip);
-                    else
-                        ex_ip_quad<ex_storage_bits(EX), 1>(uq4, row0, row0, r, D / 16, ip);
-                    if (fin) {
-                        // inc/index/HASearcher.hpp:225-232
-                        const float on = w_on[slot];
-                        const float sqr_x = __fmul_rn(on, on);
-                        const float t = __fadd_rn(__fmul_rn((float)fac_rescale, w_ipq[slot]), r == 0 ? ip[0] : ip[1]);
-                        const double br = __dsub_rn((double)t, ex_sub);
-                        const float xy = __fmul_rn(xipn, y);
-                        const float f = __fadd_rn(sqr_x, sqy);
-                        w_ed[slot] = __double2float_rn(__dsub_rn((double)f, __dmul_rn((double)xy, br)));
-                        w_id[slot] = vid;
-                    }
-                    base += step;
+                if (fin) {
+                    // inc/index/HASearcher.hpp:225-232
+                    const float y = sh.y[cs];
+                    const float ipq = __fmul_rn(__int2float_rn(sum), sh.delta[cs]);
+                    const float sqr_x = __fmul_rn(on, on);
+                    const float tt = __fadd_rn(__fmul_rn((float)(1 << EX), ipq), r == 0 ? ip[0] : ip[1]);
+                    const double br = __dsub_rn((double)tt, sh.ex_sub[cs]);
+                    const float xy = __fmul_rn(xipn, y);
+                    const float f = __fadd_rn(sqr_x, sh.sqy[cs]);
+                    sh.d[mine] = __double2float_rn(__dsub_rn((double)f, __dmul_rn((double)xy, br)));
+                    sh.id[mine] = vid;
                 }
             }
-            __syncthreads();
+        }
+        __syncthreads();
+        if (k > kSmallPool) {
             if (warp == 0) {
-                for (int b = 0; b < nbw; ++b) {
+#pragma unroll 1
+                for (int b = 0; b < nb; ++b) {
                     // candidates of the block against the threshold at its
                     // start; those above a full pool's k-th cannot enter
-                    const float ed = w_ed[32 * b + lane];
-                    const bool below = w_lb[32 * b + lane] < distk;
+                    const uint32_t m = __shfl_sync(0xffffffffu, bmask, b);
+                    const int e = __shfl_sync(0xffffffffu, end - even, b) + __popc(m & lt);
+                    const bool listed = (m >> lane) & 1u;
+                    const float d = listed ? sh.d[e] : 0.f;
+                    const bool below = listed && sh.lb[32 * b + lane] < sh.distk;
                     if (a.stats) st_cand += __popc(__ballot_sync(0xffffffffu, below));
-                    const bool enter = below && (size < k || !(ed > distk));
+                    const bool enter = below && (sh.size < k || !(d > sh.distk));
                     if (__ballot_sync(0xffffffffu, enter))
-                        pool_merge_block(pool_d, pool_id, size, k, distk, enter, ed,
-                                         w_id[32 * b + lane], cs, lane, p > 0);
-                }
-                if (lane == 0) {
-                    *s_distk = distk;
-                    misc[1] = size;
+                        pool_merge_shared(pool_d, pool_id, &sh.size, &sh.distk, k, enter, d, listed ? sh.id[e] : 0u,
+                                          sh.merge, lane, pos >= ((first_size + 31u) >> 5));
                 }
             }
-            __syncthreads();
-            wb = wnext;
+        } else if (warp == 0) {
+            rp.entries = entries;
+            if (k <= 32) replay_window<1>(rp, sp, size, worst, st_cand, lane);
+            else if (k <= 128) replay_window<4>(rp, sp, size, worst, st_cand, lane);
+            else replay_window<8>(rp, sp, size, worst, st_cand, lane);
         }
+        if (tid == 0 && k <= kSmallPool) {
+            sh.distk = order_float(worst);
+            sh.size = size;
+        }
+        __syncthreads();
+        pos = next;
     }
-    if (warp == 0) {
-        if (a.stats && lane == 0) {
-            atomicAdd(a.stats + 0, (unsigned long long)st_cand);
-            atomicAdd(a.stats + 1, (unsigned long long)st_refined);
-            atomicAdd(a.stats + 2, (unsigned long long)st_windows);
-            atomicAdd(a.stats + 3, (unsigned long long)st_blocks);
+    // the pool's entries in order: ascending distance, newer first
+    if (a.stats && tid == 0) {
+        atomicAdd(a.stats + 0, (unsigned long long)st_cand);
+        atomicAdd(a.stats + 1, (unsigned long long)st_refined);
+        atomicAdd(a.stats + 2, (unsigned long long)st_windows);
+        atomicAdd(a.stats + 3, (unsigned long long)st_blocks);
+    }
+    size = sh.size;
+    uint32_t* oid = a.out_ids + (size_t)q * k;
+    float* od = a.out_dists ? a.out_dists + (size_t)q * k : nullptr;
+    if (k > kSmallPool) {  // sorted already
+#pragma unroll 1
+        for (int i = tid; i < size; i += kThreads) {
+            oid[i] = pool_id[i];
+            if (od) od[i] = pool_d[i];
         }
-        uint32_t* oid = a.out_ids + (size_t)q * k;
-        for (int i = lane; i < k; i += 32) {
-            oid[i] = i < size ? pool_id[i] : 0u;
-            if (a.out_dists)
-                a.out_dists[(size_t)q * k + i] = i < size ? pool_d[i] : __int_as_float(0x7f800000);
-        }
+    } else if (warp == 0) {
+        if (k <= 32) pool_out<1>(sp, rp, size, oid, od, lane);
+        else if (k <= 128) pool_out<4>(sp, rp, size, oid, od, lane);
+        else pool_out<8>(sp, rp, size, oid, od, lane);
+    }
+#pragma unroll 1
+    for (int i = size + tid; i < k; i += kThreads) {
+        oid[i] = 0u;
+        if (od) od[i] = __int_as_float(0x7f800000);
     }
 }
 
