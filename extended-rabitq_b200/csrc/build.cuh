@@ -16,9 +16,10 @@
 //                         sqrt((double) that) (rabitq_factor, Quantizer.hpp:386-437)
 //   fast_quantize_kernel  the EX-bit code: fast_quantize's sweep over the
 //                         critical rescaling factors (Quantizer.hpp:138-219),
-//                         one thread per vector with its priority queue of
-//                         (t, dim) in global memory, every double step as the
-//                         reference takes it
+//                         a block per vector: windows of the factors sorted in
+//                         shared memory, every double value as the reference
+//                         computes it (fast_quantize_serial_kernel, one thread
+//                         with a heap, for vectors outside its terms)
 //   build_long_kernel     codes flipped on negative dims, store_compacted_code
 //                         (Quantizer.hpp:491-631), xipnorm = ipnorm * 2 * ||o - c||
 //   build_short_kernel    the 1-bit FastScan blocks (pack_binary + pack_codes,
@@ -148,19 +149,19 @@ __global__ void build_x2_kernel(const float* __restrict__ x, const uint32_t* __r
     }
 }
 
-// fast_quantize (inc/index/Quantizer.hpp:138-219) for rows [row0, row0 + T)
-// of xn, one thread per row.  The thread's priority queue of (t, dim),
+// fast_quantize (inc/index/Quantizer.hpp:138-219) for the rows listed in
+// list[0 .. T) of xn, one thread per row.  The thread's priority queue of (t, dim),
 // ordered by t then dim as std::priority_queue<pair, ..., greater> pops them,
 // and its current codes live in global memory, entry e of thread j at
 // e * T + j.  code[r][i] = the EX-bit magnitude code of |xn[r][i]|,
 // ipnorm[r] = 1 / sum (code + 0.5) |xn| (1 when not finite).
-__global__ void fast_quantize_kernel(const float* __restrict__ xn, int rows, int row0, int T, int D,
-                                     int EX, double* __restrict__ heap_t,
-                                     uint16_t* __restrict__ heap_i, uint8_t* __restrict__ cur,
-                                     uint8_t* __restrict__ code, float* __restrict__ ipnorm) {
+__global__ void fast_quantize_serial_kernel(const float* __restrict__ xn, const uint32_t* __restrict__ list,
+                                            int T, int D, int EX, double* __restrict__ heap_t,
+                                            uint16_t* __restrict__ heap_i, uint8_t* __restrict__ cur,
+                                            uint8_t* __restrict__ code, float* __restrict__ ipnorm) {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    const int r = row0 + j;
-    if (j >= T || r >= rows) return;
+    if (j >= T) return;
+    const size_t r = list[j];
     const float* o = xn + (size_t)r * D;
     const double eps = 1e-5;
     const int cap = (1 << EX) - 1;
@@ -257,6 +258,384 @@ __global__ void fast_quantize_kernel(const float* __restrict__ xn, int rows, int
     float ipn = __double2float_rn(__ddiv_rn(1.0, num2));
     if (!isfinite(ipn)) ipn = 1.f;
     ipnorm[r] = ipn;
+}
+
+// The same sweep, a block per vector.
+//
+// fast_quantize visits the critical factors t = c / |o_i| of all dims in
+// ascending (t, i), adds |o_i| to a numerator and 2c to a squared denominator
+// at each, and keeps the t of the first largest quotient num / sqrt(den).  The
+// block takes the factors in windows of ascending t, each bounded so that its
+// factors fit shared memory (a dim has at most w |o_i| + 1 of them in a window
+// of width w); a window is sorted by a counting sort over uniform bins of t and
+// a rank inside each bin, then the running sums are a block-wide scan and every
+// quotient is taken in parallel.
+//
+// The running numerator is a double and rounds in the reference's order.  Its
+// terms are multiples of 2^(lsb-1), lsb the last bit of the smallest non-zero
+// |o_i|: while it stays below 2^(52+lsb) no addition rounds and any order gives
+// the same doubles (and a sum in any order that ends below it was exact).  Past
+// that one thread adds in order.  The denominators are integers.  Vectors
+// without a finite positive largest |o_i|, or with more factors in a window than
+// fit, go to `slow` for the serial kernel.
+//
+// What bounds it: instructions issued (some 1700 per warp and window: counting,
+// sorting, scanning), 8 warps a block and 4 blocks an SM hiding each other's
+// barriers (4 warps a block: 12.0 ms below).  The divisions are two products
+// and four fused steps, the square roots only one per thread and window.
+// 20,000 vectors of 768 dims, EX = 7: 168.3 -> 7.0 ms (the serial kernel's heap
+// steps are chains of some 20 dependent global loads, 20,000 threads in all).
+constexpr int kFqThreads = 256;
+template <int CAP>
+struct FqShared {
+    double t[CAP];
+    union {
+        struct {
+            uint32_t bin[CAP];      // counts, then first places
+            uint16_t arrival[CAP];  // of a factor within its bin
+            uint16_t binned[CAP];   // factors by bin
+        } s;
+        double num[CAP];            // terms, then running sums, in sorted order
+    } u;
+    uint32_t item[CAP];             // dim | count << 16
+    uint16_t sorted[CAP];
+    double red[kFqThreads / 32], red2[kFqThreads / 32];
+    uint32_t scan[kFqThreads / 32], at[kFqThreads / 32];
+    double num, best, best_t;
+    uint32_t den;
+    int n, overflow;
+};
+template <int CAP>
+__host__ __device__ constexpr size_t fq_smem_bytes(int D) {
+    return sizeof(FqShared<CAP>) + (size_t)D * (8 + 4 + 2);
+}
+// CAP - D - 64 bounds a window's factors beyond one per dim
+__host__ __device__ constexpr int fq_cap(int D) { return D <= 1024 ? 2048 : 4096; }
+
+// Exclusive prefix of v over the block and its total; two barriers.
+template <typename T>
+__device__ __forceinline__ T fq_scan(T v, T* red, T* total) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    T incl = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const T x = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += x;
+    }
+    if (lane == 31) red[warp] = incl;
+    __syncthreads();
+    T before = 0, all = 0;
+#pragma unroll
+    for (int w = 0; w < kFqThreads / 32; ++w) {
+        if (w < warp) before += red[w];
+        all += red[w];
+    }
+    __syncthreads();
+    *total = all;
+    return before + incl - v;
+}
+
+// c / x correctly rounded from y = 1 / x correctly rounded, two corrected
+// steps (Markstein, IBM J. Res. Dev. 34(1), 1990); x a float, so nothing here
+// under- or overflows; c / 0 = infinity.
+__device__ __forceinline__ double fq_quotient(int c, double x, double y) {
+    const double a = (double)c;
+    double q = __dmul_rn(a, y);
+    if (x > 0.0) {
+        q = __fma_rn(__fma_rn(-x, q, a), y, q);
+        q = __fma_rn(__fma_rn(-x, q, a), y, q);
+    }
+    return q;
+}
+
+template <int CAP>
+__global__ void __launch_bounds__(kFqThreads) fast_quantize_kernel(const float* __restrict__ xn, int rows, int D,
+                                                                   int EX, uint8_t* __restrict__ code,
+                                                                   float* __restrict__ ipnorm,
+                                                                   uint32_t* __restrict__ slow,
+                                                                   uint32_t* __restrict__ slow_n) {
+    extern __shared__ __align__(16) uint8_t smem_raw[];
+    FqShared<CAP>& sh = *reinterpret_cast<FqShared<CAP>*>(smem_raw);
+    double* inv = reinterpret_cast<double*>(smem_raw + sizeof(FqShared<CAP>));  // 1 / |o_i|
+    float* v = reinterpret_cast<float*>(inv + D);
+    uint16_t* cn = reinterpret_cast<uint16_t*>(v + D);  // count at the next factor of a dim, 0: none left
+    const int r = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const float* o = xn + (size_t)r * D;
+    const double eps = 1e-5;
+    const int cap = (1 << EX) - 1;
+    // largest, smallest non-zero, sum
+    float mx = 0.f, mn = INFINITY;
+    double sum = 0.0;
+    bool finite = true;
+    for (int i = tid; i < D; i += kFqThreads) {
+        const float x = fabsf(o[i]);
+        v[i] = x;
+        finite = finite && x < INFINITY;  // false for NaN
+        mx = fmaxf(mx, x);
+        if (x > 0.f) mn = fminf(mn, x);
+        sum += (double)x;
+    }
+    mx = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(mx)));
+    mn = __uint_as_float(__reduce_min_sync(0xffffffffu, __float_as_uint(mn)));
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, s);
+    if (lane == 0) {
+        sh.red[warp] = sum;
+        sh.scan[warp] = __float_as_uint(mx);
+        sh.at[warp] = __float_as_uint(mn);
+    }
+    if (tid == 0) {
+        sh.n = 0;
+        sh.overflow = 0;
+        sh.best = 0.0;
+        sh.best_t = 0.0;
+    }
+    finite = __syncthreads_and(finite);
+    sum = 0.0;
+#pragma unroll
+    for (int w = 0; w < kFqThreads / 32; ++w) {
+        sum += sh.red[w];
+        mx = fmaxf(mx, __uint_as_float(sh.scan[w]));
+        mn = fminf(mn, __uint_as_float(sh.at[w]));
+    }
+    const double t_start = __ddiv_rn((double)(cap / 3), (double)mx);
+    const double t_end = __ddiv_rn((double)(cap + 10), (double)mx);
+    if (!finite || !(mx > 0.f) || !(t_end < 1e300)) {  // uniform
+        if (tid == 0) slow[atomicAdd(slow_n, 1u)] = (uint32_t)r;
+        return;
+    }
+    const int lsb = max((int)(__float_as_uint(mn) >> 23), 1) - 127 - 23;
+    const double limit = __longlong_as_double((long long)(52 + lsb + 1023) << 52);  // sums below are exact
+    __syncthreads();  // red, scan and at are reused
+    // the state at t_start
+    double num0 = 0.0;
+    uint32_t den0 = 0;
+    for (int i = tid; i < D; i += kFqThreads) {
+        const double x = (double)v[i];
+        const int c = __double2int_rz(__dadd_rn(__dmul_rn(t_start, x), eps));
+        const double term = __dmul_rn((double)c + 0.5, x);
+        num0 = __dadd_rn(num0, term);
+        sh.u.num[i] = term;
+        den0 += (uint32_t)(c * c + c);
+        inv[i] = __drcp_rn(x);
+        cn[i] = (uint16_t)(c + 1);
+    }
+    {
+        double all = 0.0;
+        uint32_t alld = 0;
+        fq_scan<double>(num0, sh.red, &all);
+        fq_scan<uint32_t>(den0, sh.scan, &alld);
+        if (tid == 0) {
+            if (!(all < limit)) {
+                all = 0.0;
+                for (int i = 0; i < D; ++i) all = __dadd_rn(all, sh.u.num[i]);
+            }
+            sh.num = all;
+            sh.den = alld + (uint32_t)(D / 4);
+        }
+    }
+    const double width = (double)(CAP - D - 64) / sum;
+    double lo = t_start;
+    for (bool tail = false;;) {
+        const double hi = tail ? INFINITY : fmin(lo + width, t_end);
+        const double scale = (double)CAP / width;
+        // the bin of a factor (non-decreasing in t); past t_end, 32 per octave
+        const auto bin_of = [&](double t) -> int {
+            if (tail) {
+                const long long d = (__double_as_longlong(t) - __double_as_longlong(t_end)) >> 47;
+                return (int)(d < 0 ? 0 : (d < CAP ? d : CAP - 1));
+            }
+            const int b = __double2int_rz((t - lo) * scale);
+            return b < 0 ? 0 : (b < CAP ? b : CAP - 1);
+        };
+        __syncthreads();  // the window before has been read
+        for (int b = tid; b < CAP; b += kFqThreads) sh.u.s.bin[b] = 0u;
+        __syncthreads();
+        // this window's factors: counted by dim, listed, then placed one by one
+        for (int i0 = 0; i0 < D; i0 += kFqThreads) {
+            const int i = i0 + tid, c0 = i < D ? cn[i] : 0;
+            int m = 0;
+            if (c0 > 0) {
+                const double x = (double)v[i], y = inv[i];
+                if (tail) {
+                    m = 1;
+                } else {
+                    int last = min(__double2int_rz(hi * x) + 1, cap);
+                    while (last >= c0 && !(fq_quotient(last, x, y) < hi)) --last;
+                    m = max(last + 1 - c0, 0);
+                    if (m > 0) cn[i] = last < cap && fq_quotient(last + 1, x, y) < t_end ? last + 1 : 0;
+                }
+            }
+            int incl = m;
+#pragma unroll
+            for (int s = 1; s < 32; s <<= 1) {
+                const int x = __shfl_up_sync(0xffffffffu, incl, s);
+                if (lane >= s) incl += x;
+            }
+            int at = 0;
+            if (lane == 31 && incl > 0) at = atomicAdd(&sh.n, incl);
+            at = __shfl_sync(0xffffffffu, at, 31) + incl - m;
+            for (int j = 0; j < m && at + j < CAP; ++j)
+                sh.item[at + j] = (uint32_t)i | ((uint32_t)(c0 + j) << 16);
+        }
+        __syncthreads();
+        const int n = sh.n;
+        if (n > CAP) {  // uniform
+            if (tid == 0) slow[atomicAdd(slow_n, 1u)] = (uint32_t)r;
+            return;
+        }
+        for (int e = tid; e < n; e += kFqThreads) {
+            const uint32_t it = sh.item[e], i = it & 0xffffu;
+            const double t = fq_quotient((int)(it >> 16), (double)v[i], inv[i]);
+            sh.t[e] = t;
+            sh.u.s.arrival[e] = (uint16_t)atomicAdd(&sh.u.s.bin[bin_of(t)], 1u);
+        }
+        __syncthreads();
+        // first places of the bins
+        {
+            constexpr int PER = CAP / kFqThreads / 4;
+            uint4* mine = reinterpret_cast<uint4*>(sh.u.s.bin) + tid * PER;
+            uint4 c[PER];
+            uint32_t own = 0, all = 0;
+#pragma unroll
+            for (int b = 0; b < PER; ++b) {
+                c[b] = mine[b];
+                own += c[b].x + c[b].y + c[b].z + c[b].w;
+            }
+            uint32_t run = fq_scan<uint32_t>(own, sh.scan, &all);
+#pragma unroll
+            for (int b = 0; b < PER; ++b) {
+                uint4 f;
+                f.x = run;
+                f.y = f.x + c[b].x;
+                f.z = f.y + c[b].y;
+                f.w = f.z + c[b].z;
+                run = f.w + c[b].w;
+                mine[b] = f;
+            }
+        }
+        __syncthreads();
+        for (int e = tid; e < n; e += kFqThreads)
+            sh.u.s.binned[sh.u.s.bin[bin_of(sh.t[e])] + sh.u.s.arrival[e]] = (uint16_t)e;
+        __syncthreads();
+        // a factor's rank within its bin, by (t, dim)
+        for (int e = tid; e < n; e += kFqThreads) {
+            const double t = sh.t[e];
+            const int b = bin_of(t);
+            const uint32_t first = sh.u.s.bin[b], last = b + 1 < CAP ? sh.u.s.bin[b + 1] : (uint32_t)n;
+            const uint32_t dim = sh.item[e] & 0xffffu;
+            uint32_t at = first;
+            for (uint32_t k = first; k < last; ++k) {
+                const int f = sh.u.s.binned[k];
+                at += sh.t[f] < t || (sh.t[f] == t && (sh.item[f] & 0xffffu) < dim);
+            }
+            sh.sorted[at] = (uint16_t)e;
+        }
+        __syncthreads();
+        // running sums and quotients, each thread a stretch of the sequence
+        const int per = (n + kFqThreads - 1) / kFqThreads;
+        const int k0 = min(n, tid * per), k1 = min(n, k0 + per);
+        double own = 0.0;
+        uint32_t ownd = 0;
+        for (int k = k0; k < k1; ++k) {
+            const uint32_t it = sh.item[sh.sorted[k]];
+            const double x = (double)v[it & 0xffffu];
+            sh.u.num[k] = x;
+            own = __dadd_rn(own, x);
+            ownd += 2u * (it >> 16);
+        }
+        double all = 0.0;
+        uint32_t alld = 0;
+        double num = fq_scan<double>(own, sh.red, &all);
+        uint32_t den = fq_scan<uint32_t>(ownd, sh.scan, &alld) + sh.den;
+        num = __dadd_rn(num, sh.num);
+        all = __dadd_rn(all, sh.num);
+        const bool exact = all < limit;
+        if (!exact) {  // uniform: in order, by one thread
+            if (tid == 0) {
+                double x = sh.num;
+#pragma unroll 4
+                for (int k = 0; k < n; ++k) {
+                    x = __dadd_rn(x, sh.u.num[k]);
+                    sh.u.num[k] = x;
+                }
+                all = x;
+            }
+            __syncthreads();
+        }
+        // The squared quotients compared by their cross products: where those
+        // differ by 1e-14, some 20 times what the rounded quotient can be off,
+        // the rounded quotients are in the same order.
+        double bnum = 0.0, bden = 1.0;
+        int best_k = -1;
+        for (int k = k0; k < k1; ++k) {
+            num = exact ? __dadd_rn(num, sh.u.num[k]) : sh.u.num[k];
+            den += 2u * (sh.item[sh.sorted[k]] >> 16);
+            const double a = num * num * bden, b = bnum * bnum * (double)den;
+            bool more = a > b;
+            if (fabs(a - b) <= 1e-14 * b)
+                more = __ddiv_rn(num, __dsqrt_rn((double)den)) > __ddiv_rn(bnum, __dsqrt_rn(bden));
+            if (more) {
+                bnum = num;
+                bden = (double)den;
+                best_k = k;
+            }
+        }
+        double best = best_k < 0 ? -1.0 : __ddiv_rn(bnum, __dsqrt_rn(bden));
+        // the first largest quotient of the window
+#pragma unroll
+        for (int s = 16; s > 0; s >>= 1) {
+            const double ob = __shfl_xor_sync(0xffffffffu, best, s);
+            const int ok = __shfl_xor_sync(0xffffffffu, best_k, s);
+            if (ob > best || (ob == best && ok < best_k)) {
+                best = ob;
+                best_k = ok;
+            }
+        }
+        if (lane == 0) {
+            sh.red2[warp] = best;
+            sh.at[warp] = (uint32_t)best_k;
+        }
+        __syncthreads();  // sh.num and sh.den have been read
+        if (tid == 0) {
+#pragma unroll
+            for (int w = 0; w < kFqThreads / 32; ++w)  // the warps' stretches are in order
+                if (sh.red2[w] > sh.best) {
+                    sh.best = sh.red2[w];
+                    sh.best_t = sh.t[sh.sorted[sh.at[w]]];
+                }
+            sh.num = all;
+            sh.den += alld;
+            sh.n = 0;
+        }
+        if (tail) break;
+        tail = hi >= t_end;
+        lo = hi;
+    }
+    __syncthreads();
+    // the codes at the best factor, and 1 / sum (code + 0.5) |o|
+    const double t = sh.best_t;
+    uint8_t* out = code + (size_t)r * D;
+    double own = 0.0, all = 0.0;
+    for (int i = tid; i < D; i += kFqThreads) {
+        const double x = (double)v[i];
+        int b = __double2int_rz(__dadd_rn(__dmul_rn(t, x), eps));
+        if (b >= (1 << EX)) b = cap;
+        const double term = __dmul_rn((double)b + 0.5, x);
+        own = __dadd_rn(own, term);
+        sh.u.num[i] = term;
+        out[i] = (uint8_t)b;
+    }
+    fq_scan<double>(own, sh.red, &all);
+    if (tid == 0) {
+        if (!(all < limit)) {
+            all = 0.0;
+            for (int i = 0; i < D; ++i) all = __dadd_rn(all, sh.u.num[i]);
+        }
+        float ipn = __double2float_rn(__ddiv_rn(1.0, all));
+        if (!isfinite(ipn)) ipn = 1.f;
+        ipnorm[r] = ipn;
+    }
 }
 
 // Per row: codes flipped where the sign bit is 0, compacted to D*EX/8 bytes

@@ -2771,17 +2771,37 @@ erq_status erq_build_index(const float* data, uint64_t n, uint64_t dim, const fl
     build_rows_kernel<<<(unsigned)div_up(n, 128), 128>>>(xp, (int)n, (int)D, bits);
     ERQ_CUDA(cudaGetLastError());
     {
-        const uint64_t T = std::min<uint64_t>(n, 65536);
-        double* ht = nullptr;
-        uint16_t* hi = nullptr;
-        uint8_t* cur = nullptr;
-        ERQ_TRY(b.alloc(&ht, T * D));
-        ERQ_TRY(b.alloc(&hi, T * D));
-        ERQ_TRY(b.alloc(&cur, T * D));
-        for (uint64_t r0 = 0; r0 < n; r0 += T) {
-            fast_quantize_kernel<<<(unsigned)div_up(T, 128), 128>>>(xp, (int)n, (int)r0, (int)T, (int)D,
-                                                                    (int)EX, ht, hi, cur, code, ipn);
-            ERQ_CUDA(cudaGetLastError());
+        uint32_t *slow = nullptr, *slow_n = nullptr;
+        ERQ_TRY(b.alloc(&slow, n));
+        ERQ_TRY(b.alloc(&slow_n, 1));
+        ERQ_CUDA(cudaMemset(slow_n, 0, sizeof(uint32_t)));
+        ERQ_CUDA(cudaFuncSetAttribute(fast_quantize_kernel<2048>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)fq_smem_bytes<2048>(1024)));
+        ERQ_CUDA(cudaFuncSetAttribute(fast_quantize_kernel<4096>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)fq_smem_bytes<4096>(kMaxD)));
+        if (fq_cap((int)D) == 2048)
+            fast_quantize_kernel<2048><<<(unsigned)n, kFqThreads, fq_smem_bytes<2048>((int)D)>>>(
+                xp, (int)n, (int)D, (int)EX, code, ipn, slow, slow_n);
+        else
+            fast_quantize_kernel<4096><<<(unsigned)n, kFqThreads, fq_smem_bytes<4096>((int)D)>>>(
+                xp, (int)n, (int)D, (int)EX, code, ipn, slow, slow_n);
+        ERQ_CUDA(cudaGetLastError());
+        uint32_t left = 0;  // vectors the block form leaves to the serial one
+        ERQ_CUDA(cudaMemcpy(&left, slow_n, sizeof(left), cudaMemcpyDeviceToHost));
+        if (left) {
+            const uint64_t T = std::min<uint64_t>(left, 65536);
+            double* ht = nullptr;
+            uint16_t* hi = nullptr;
+            uint8_t* cur = nullptr;
+            ERQ_TRY(b.alloc(&ht, T * D));
+            ERQ_TRY(b.alloc(&hi, T * D));
+            ERQ_TRY(b.alloc(&cur, T * D));
+            for (uint64_t r0 = 0; r0 < left; r0 += T) {
+                const int m = (int)std::min<uint64_t>(T, left - r0);
+                fast_quantize_serial_kernel<<<(unsigned)div_up(m, 128), 128>>>(xp, slow + r0, m, (int)D, (int)EX,
+                                                                              ht, hi, cur, code, ipn);
+                ERQ_CUDA(cudaGetLastError());
+            }
         }
     }
     build_long_kernel<<<(unsigned)div_up(n * (D / 64), 128), 128>>>(code, bits, ipn, onorm, (int)n, (int)D,
