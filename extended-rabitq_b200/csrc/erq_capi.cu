@@ -289,6 +289,15 @@ erq_status dev_alloc(erq_index* idx, T** p, size_t count) {
     return ERQ_OK;
 }
 
+// The split of R rows (gemm.cuh); by warps where a row fits one.
+void split_rows(const float* in, int R, int C, int Cp, bool a_side, __nv_bfloat16* out, float* norms,
+                cudaStream_t st) {
+    if (Cp <= 256)
+        split_rows_warp_kernel<<<(unsigned)div_up(R, 8), 256, 0, st>>>(in, R, C, Cp, a_side, out, norms);
+    else
+        split_rows_kernel<<<(unsigned)R, 256, 0, st>>>(in, R, C, Cp, a_side, out, norms);
+}
+
 erq_status load_impl(const char* path, erq_index* idx) {
     std::unique_ptr<FILE, FileCloser> f(fopen(path, "rb"));
     if (!f) return fail(ERQ_ERR_IO, "cannot open index file '%s'", path);
@@ -464,10 +473,8 @@ erq_status load_impl(const char* path, erq_index* idx) {
         ERQ_CUDA(cudaMalloc(&tmp, D * D * 4));
         cudaError_t e = cudaMemcpy(tmp, hpt.data(), D * D * 4, cudaMemcpyHostToDevice);
         if (e == cudaSuccess) {
-            split_rows_kernel<<<(unsigned)D, 256>>>(tmp, (int)D, (int)D, (int)D, false,
-                                                    idx->pt_split, nullptr);
-            split_rows_kernel<<<(unsigned)K, 256>>>(idx->centroids, (int)K, (int)D, (int)D, false,
-                                                    idx->c_split, idx->cn);
+            split_rows(tmp, (int)D, (int)D, (int)D, false, idx->pt_split, nullptr, nullptr);
+            split_rows(idx->centroids, (int)K, (int)D, (int)D, false, idx->c_split, idx->cn, nullptr);
             chain_layout_kernel<<<1184, 256>>>(idx->centroids, (int)K, (int)D, idx->c_chain);
             e = cudaGetLastError();
             if (e == cudaSuccess) e = cudaDeviceSynchronize();
@@ -686,8 +693,9 @@ erq_status gemm_tc(const __nv_bfloat16* A, const __nv_bfloat16* B, float* C, int
         ERQ_CUDA(cudaGetDevice(&dev));
         std::lock_guard<std::mutex> g(mu);
         if (!configured[dev]) {
-            ERQ_CUDA(cudaFuncSetAttribute(gemm_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)gemm_tc_smem_bytes()));
+            for (auto kernel : {gemm_tc_kernel<false>, gemm_tc_kernel<true>})
+                ERQ_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                              (int)gemm_tc_smem_bytes()));
             configured[dev] = true;
         }
     }
@@ -696,8 +704,9 @@ erq_status gemm_tc(const __nv_bfloat16* A, const __nv_bfloat16* B, float* C, int
     if (tiles > 0x7fffffffull) return fail(ERQ_ERR_INVALID_ARGUMENT, "GEMM of %llu tiles", (unsigned long long)tiles);
     const unsigned grid = (unsigned)std::min<uint64_t>(tiles, (uint64_t)device_sms());
     LaunchTimer t(kernel_id, st);
-    gemm_tc_kernel<<<grid, kTcThreads, gemm_tc_smem_bytes(), st>>>(ta, tb, C, M, N, Kd, epi, status,
-                                                                    g_tc_wait_limit.load());
+    const auto kernel = epi.nearest ? gemm_tc_kernel<true> : gemm_tc_kernel<false>;
+    kernel<<<grid, kTcThreads, gemm_tc_smem_bytes(), st>>>(ta, tb, C, M, N, Kd, epi, status,
+                                                           g_tc_wait_limit.load());
     t.finish();
     ERQ_CUDA(cudaGetLastError());
     return ERQ_OK;
@@ -990,8 +999,7 @@ erq_status launch_probe_tc(const erq_index* idx, const Batch& b, uint64_t nprobe
     if (split) *split = false;
     {
         LaunchTimer t(kSplit, st);
-        split_rows_kernel<<<(unsigned)b.nq, 256, 0, st>>>(b.qrot, (int)b.nq, D, D, true, b.qsplit,
-                                                          b.qn);
+        split_rows(b.qrot, (int)b.nq, D, D, true, b.qsplit, b.qn, st);
         t.finish();
         ERQ_CUDA(cudaGetLastError());
     }
@@ -1424,8 +1432,7 @@ erq_status rotate_into(const erq_index* idx, const float* q_dev, uint64_t nq, fl
     const int D = (int)idx->D;
     {
         LaunchTimer t(kSplit, st);
-        split_rows_kernel<<<(unsigned)nq, 256, 0, st>>>(q_dev, (int)nq, (int)idx->DIM, D, true, qs,
-                                                        nullptr);
+        split_rows(q_dev, (int)nq, (int)idx->DIM, D, true, qs, nullptr, st);
         t.finish();
         ERQ_CUDA(cudaGetLastError());
     }
@@ -1791,18 +1798,22 @@ erq_status km_iterate(const float* x, uint64_t n, uint64_t dim, uint64_t k, int 
                       uint32_t* assign, uint64_t& rng, uint32_t* counts_host, bool final_assign,
                       cudaStream_t st) {
     const uint64_t Cp = (dim + 63) / 64 * 64;
-    const uint64_t R = std::min<uint64_t>(n, std::max<uint64_t>(1024, (256ull << 20) / std::max<uint64_t>(k, 1)));
+    // Rows split at a time: what fits the memory of 256 Mi distances (float) and
+    // the splits of as many rows as those distances stand for.  When that is all
+    // of x it is split once, not in each iteration.
+    const uint64_t rows_d = std::min<uint64_t>(n, std::max<uint64_t>(1024, (256ull << 20) / std::max<uint64_t>(k, 1)));
+    const uint64_t R = std::min<uint64_t>(n, std::max(rows_d, rows_d * (4 * k + 6 * Cp + 4) / (6 * Cp + 12)));
     KmBuffers b;
     __nv_bfloat16 *c_split = nullptr, *x_split = nullptr;
-    float *cn = nullptr, *xn = nullptr, *dist = nullptr;
-    unsigned long long* sums = nullptr;
+    float *cn = nullptr, *xn = nullptr;
+    unsigned long long *sums = nullptr, *nearest = nullptr;
     uint32_t* counts = nullptr;
     unsigned* amax = nullptr;
     ERQ_TRY(b.alloc(&c_split, k * 3 * Cp));
     ERQ_TRY(b.alloc(&cn, k));
     ERQ_TRY(b.alloc(&x_split, R * 3 * Cp));
     ERQ_TRY(b.alloc(&xn, R));
-    ERQ_TRY(b.alloc(&dist, R * k));
+    ERQ_TRY(b.alloc(&nearest, R));
     ERQ_TRY(b.alloc(&sums, k * dim));
     ERQ_TRY(b.alloc(&counts, k));
     ERQ_TRY(b.alloc(&amax, 1));
@@ -1818,20 +1829,24 @@ erq_status km_iterate(const float* x, uint64_t n, uint64_t dim, uint64_t k, int 
     const double top = std::max(1e-30, (double)amax_f) * (double)n;
     const double scale = std::ldexp(1.0, std::min(32, (int)std::floor(61.0 - std::log2(top))));
     std::vector<uint32_t> cnt(k);
+    ERQ_CUDA(cudaMemsetAsync(nearest, 0xff, R * sizeof(unsigned long long), st));
+    bool split = false;  // x_split holds all of x
     auto assign_all = [&]() -> erq_status {
-        split_rows_kernel<<<(unsigned)k, 256, 0, st>>>(cent, (int)k, (int)dim, (int)Cp, false, c_split, cn);
+        split_rows(cent, (int)k, (int)dim, (int)Cp, false, c_split, cn, st);
         ERQ_CUDA(cudaGetLastError());
         for (uint64_t r0 = 0; r0 < n; r0 += R) {
             const uint64_t rows = std::min(R, n - r0);
-            split_rows_kernel<<<(unsigned)rows, 256, 0, st>>>(x + r0 * dim, (int)rows, (int)dim, (int)Cp,
-                                                              true, x_split, xn);
-            ERQ_CUDA(cudaGetLastError());
+            if (!split) {
+                split_rows(x + r0 * dim, (int)rows, (int)dim, (int)Cp, true, x_split, xn, st);
+                ERQ_CUDA(cudaGetLastError());
+                split = rows == n;
+            }
             GemmEpilogue epi;
             epi.row_norm = xn;
             epi.col_norm = cn;
-            ERQ_TRY(gemm_tc(x_split, c_split, dist, (int)rows, (int)k, (int)(3 * Cp), epi, kGemm, st));
-            argmin_rows_kernel<<<(unsigned)div_up(rows * 32, 256), 256, 0, st>>>(dist, (int)rows, (int)k,
-                                                                                 assign + r0);
+            epi.nearest = nearest;
+            ERQ_TRY(gemm_tc(x_split, c_split, nullptr, (int)rows, (int)k, (int)(3 * Cp), epi, kGemm, st));
+            take_nearest_kernel<<<(unsigned)div_up(rows, 256), 256, 0, st>>>(nearest, (int)rows, assign + r0);
             ERQ_CUDA(cudaGetLastError());
         }
         return ERQ_OK;

@@ -12,8 +12,9 @@
 //            issues tcgen05.mma.cta_group::1.kind::f16 (M 128, N 256, K 16)
 //            four times per slice into the accumulator of the tile, frees
 //            each slot with tcgen05.commit, and commits the accumulator;
-//   warps 2-5              read an accumulator back (tcgen05.ld 32x32b, each
-//            warp the 32 TMEM lanes of its quadrant), release it, and apply
+//   warps 2-9              read an accumulator back (tcgen05.ld 32x32b, each
+//            warp the 32 TMEM lanes of its quadrant in half of the columns,
+//            so that two warps hide each other's latencies), release it, and apply
 //            the epilogue of gemm.cuh (plain, distance ranking, bias + ReLU)
 //            while the MMAs of the next tile fill the other accumulator.
 // Barriers: full/empty per ring slot, tfull/tempty per accumulator, and a
@@ -32,7 +33,8 @@
 namespace erq {
 
 constexpr int kTcBM = 128, kTcBN = 256, kTcBK = 64, kTcStages = 4;
-constexpr int kTcThreads = 192;
+constexpr int kTcThreads = 320;
+constexpr int kTcEpiWarps = kTcThreads / 32 - 2;  // two per TMEM lane quadrant, half of the columns each
 constexpr uint32_t kTcABytes = kTcBM * kTcBK * 2;   // 16 KB
 constexpr uint32_t kTcBBytes = kTcBN * kTcBK * 2;   // 32 KB
 constexpr uint32_t kTcStageBytes = kTcABytes + kTcBBytes;
@@ -68,30 +70,34 @@ __device__ __forceinline__ void tc_fence_after() {
 
 constexpr int kTpAccumCols = 256;  // columns per accumulator (two of them)
 
-// A warp's 32 x 32 block of the accumulator on its way to memory.  The pitch
-// puts the 16-byte pieces of 8 rows in different banks.
-constexpr int kTcPitch = 36;
-constexpr size_t kTcSlabBytes = 32 * kTcPitch * sizeof(float);
+// A warp's 32 x 32 block of the accumulator on its way to memory, the 16-byte
+// piece p of row r at p ^ (r & 7): 8 rows' pieces are in different banks.
+constexpr size_t kTcSlabBytes = 32 * 32 * sizeof(float);
+__device__ __forceinline__ float* tc_slab_at(float* slab, int r, int p) {
+    return slab + 32 * r + 4 * (p ^ (r & 7));
+}
 
 // 1024 bytes of alignment slack + the ring + barriers and the TMEM address +
 // the epilogue warps' blocks
 __host__ __device__ constexpr size_t gemm_tc_smem_bytes() {
-    return 1024 + (size_t)kTcStages * kTcStageBytes + 256 + 4 * kTcSlabBytes;
+    return 1024 + (size_t)kTcStages * kTcStageBytes + 256 + kTcEpiWarps * kTcSlabBytes;
 }
 
 // Rows row0 .. row0+31 and columns col0 .. col0+31 of the output, lane l
 // holding row row0 + l.  The block is turned around in shared memory, so that 8
 // lanes store 128 contiguous bytes of a row and the norms are read once per
-// block: stored as held, each instruction wrote 16 bytes of 32 rows.  10,000 x
-// 4096 x 4608: 307 -> 290 us; 10,000 x 1536 x 4608: 135 -> 128.6 us; 2000 x 4096 x
-// 4608: 83 -> 76 us; 1000 x 1024 x 384: 25 -> 21 us.
+// block: stored as held, each instruction wrote 16 bytes of 32 rows.  With four
+// warps as held, four turned around, eight turned around: 10,000 x 4096 x 4608
+// 307, 290, 283 us; 10,000 x 1536 x 4608 135, 128.6, 125 us; 2000 x 4096 x 4608 83,
+// 76, 72 us; 1000 x 1024 x 384 25, 21, 16.8 us.
 __device__ __forceinline__ void gemm_epilogue_store(const uint32_t (&v)[32], float* slab,
                                                     float* __restrict__ Cout, int M, int N, int row0,
                                                     int col0, const GemmEpilogue& epi) {
     const int lane = threadIdx.x & 31;
 #pragma unroll
     for (int j = 0; j < 32; j += 4)
-        *reinterpret_cast<uint4*>(slab + lane * kTcPitch + j) = make_uint4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+        *reinterpret_cast<uint4*>(tc_slab_at(slab, lane, j / 4)) =
+            make_uint4(v[j], v[j + 1], v[j + 2], v[j + 3]);
     __syncwarp();
     const int col = col0 + 4 * (lane & 7);
     float cn[4], bias[4];
@@ -106,7 +112,7 @@ __device__ __forceinline__ void gemm_epilogue_store(const uint32_t (&v)[32], flo
     for (int i = 0; i < 8; ++i) {
         const int lr = 4 * i + (lane >> 3), row = row0 + lr;
         if (row >= M) continue;
-        const float4 y = *reinterpret_cast<const float4*>(slab + lr * kTcPitch + 4 * (lane & 7));
+        const float4 y = *reinterpret_cast<const float4*>(tc_slab_at(slab, lr, lane & 7));
         float x[4] = {y.x, y.y, y.z, y.w};
         const float rn = epi.row_norm ? epi.row_norm[row] : 0.f;
 #pragma unroll
@@ -127,6 +133,54 @@ __device__ __forceinline__ void gemm_epilogue_store(const uint32_t (&v)[32], flo
     __syncwarp();
 }
 
+// The norms of columns col0 .. col0+31 (infinity past the last), asked for before
+// the accumulator is read so that the two waits overlap.
+__device__ __forceinline__ void load_col_norms(const float* __restrict__ col_norm, int N, int col0,
+                                               float (&cn)[32]) {
+    if (col0 + 31 < N) {
+#pragma unroll
+        for (int j = 0; j < 32; j += 4) {
+            const float4 c = __ldg(reinterpret_cast<const float4*>(col_norm + col0 + j));
+            cn[j] = c.x, cn[j + 1] = c.y, cn[j + 2] = c.z, cn[j + 3] = c.w;
+        }
+    } else {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) cn[j] = col0 + j < N ? __ldg(col_norm + col0 + j) : INFINITY;
+    }
+}
+
+// The smallest ranking value of columns col0 .. col0+31 and its column (the
+// first of equal ones), on top of (best, at) of the columns before, for the row
+// this lane holds.  The minimum of the 32 is a tree; its column is looked for
+// only where some row's minimum fell.
+__device__ __forceinline__ void gemm_epilogue_nearest(const uint32_t (&v)[32], const float (&cn)[32], int col0,
+                                                      float rn, float& best, int& at) {
+    float x[32], m[4];
+#pragma unroll
+    for (int j = 0; j < 32; j += 4) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            x[j + e] = rn + cn[j + e] - 2.f * __uint_as_float(v[j + e]);
+            m[e] = j ? fminf(m[e], x[j + e]) : x[j + e];
+        }
+    }
+    const float least = fminf(fminf(m[0], m[1]), fminf(m[2], m[3]));
+    const bool less = least < best;
+    if (!__any_sync(0xffffffffu, less)) return;
+    int c = 0;
+#pragma unroll
+    for (int j = 31; j >= 0; --j) c = x[j] == least ? j : c;
+    if (less) {
+        best = least;
+        at = col0 + c;
+    }
+}
+
+// NEAREST: the epilogue keeps each row's smallest ranking value instead of
+// storing the block (kmeans.cuh).  200,000 x 1024 x 128 dims: the 819 MB of
+// rankings cost 680 us to write and 116 us to read for the minimum; this takes 148
+// us (with the four warps and the serial minimum that were tried first, 252).
+template <bool NEAREST>
 __global__ void __launch_bounds__(kTcThreads, 1) gemm_tc_kernel(
     const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
     float* __restrict__ Cout, int M, int N, int Kd, GemmEpilogue epi, uint32_t* status,
@@ -151,7 +205,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemm_tc_kernel(
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(tfull0 + 8 * b, 1);
-            mbar_init(tempty0 + 8 * b, 4);  // one arrival per epilogue warp
+            mbar_init(tempty0 + 8 * b, kTcEpiWarps);  // one arrival per epilogue warp
         }
         mbar_init(drain, 1);
         *flag = 0u;
@@ -243,18 +297,25 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemm_tc_kernel(
         }
     } else {
         const int q = warp & 3;  // TMEM lane quadrant this warp may read
-        float* slab = reinterpret_cast<float*>(smem_raw + (bars + 256 - raw) + q * kTcSlabBytes);
+        const int cb = warp < 6 ? 0 : kTcBN / 2;  // its columns of the tile
+        float* slab = reinterpret_cast<float*>(smem_raw + (bars + 256 - raw) + (warp - 2) * kTcSlabBytes);
         int i = 0;
         for (int t = blockIdx.x; t < tiles; t += gridDim.x, ++i) {
             const int b = i & 1;
             const uint32_t u = (uint32_t)(i >> 1);
+            const int m0 = (t / tiles_n) * kTcBM, n0 = (t % tiles_n) * kTcBN;
+            const int row = m0 + 32 * q + lane;
+            const float rn = NEAREST && row < M ? epi.row_norm[row] : 0.f;
             if (!mbar_wait(tfull0 + 8 * b, u & 1u, wait_limit) || *flag) {
                 *flag = 1u;
                 break;
             }
             tc_fence_after();
-            const int m0 = (t / tiles_n) * kTcBM, n0 = (t % tiles_n) * kTcBN;
-            for (int c0 = 0; c0 < kTcBN; c0 += 32) {
+            float best = INFINITY;
+            int at = 0;
+            for (int c0 = cb; c0 < cb + kTcBN / 2; c0 += 32) {
+                float cn[32];
+                if constexpr (NEAREST) load_col_norms(epi.col_norm, N, n0 + c0, cn);
                 uint32_t v[32];
                 const uint32_t taddr = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(b * kTpAccumCols + c0);
                 asm volatile(
@@ -268,13 +329,19 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemm_tc_kernel(
                       "=r"(v[31])
                     : "r"(taddr));
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                if (c0 + kTcBN / 8 >= kTcBN) {
+                if (c0 + 32 >= cb + kTcBN / 2) {
                     // the last columns are in registers: the accumulator is free
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) mbar_arrive(tempty0 + 8 * b);
                 }
-                gemm_epilogue_store(v, slab, Cout, M, N, m0 + 32 * q, n0 + c0, epi);
+                if constexpr (NEAREST) gemm_epilogue_nearest(v, cn, n0 + c0, rn, best, at);
+                else gemm_epilogue_store(v, slab, Cout, M, N, m0 + 32 * q, n0 + c0, epi);
+            }
+            if (NEAREST && row < M && best < INFINITY) {
+                const uint32_t u = __float_as_uint(best + 0.f);  // -0 orders as 0
+                const uint32_t key = u ^ ((u >> 31) ? 0xffffffffu : 0x80000000u);
+                atomicMin(epi.nearest + row, ((unsigned long long)key << 32) | (uint32_t)at);
             }
         }
     }

@@ -9,10 +9,11 @@
 // dimension, eps = 1/1024, and the points are shared).
 //
 // Here one iteration is
-//   1. distance ranks ||x||^2 + ||c||^2 - 2 x.c on the tensor cores (the
-//      split-BF16 GEMM of gemm_tc.cuh, about FP32 accuracy), in row chunks;
-//   2. argmin_rows_kernel: the nearest centroid of each point (ties: the
-//      smaller index);
+//   1. the nearest centroid of each point: distance ranks ||x||^2 + ||c||^2 -
+//      2 x.c on the tensor cores (the split-BF16 GEMM of gemm_tc.cuh, about FP32
+//      accuracy), whose epilogue keeps the smallest rank of a row (ties: the
+//      smaller index) in 64-bit atomic minima of (rank, column);
+//   2. take_nearest_kernel: the columns of the minima;
 //   3. kmeans_accumulate_kernel: per-cluster sums in 64-bit fixed point
 //      (scale 2^s, s <= 32 chosen so that n * max|x| * 2^s < 2^62), so the
 //      integer atomics give the same sums in any order and the clustering is
@@ -27,32 +28,15 @@
 
 namespace erq {
 
-// One warp per row of dist [rows][K]: the column of the smallest value
-// (smallest index among equal ones).
-__global__ void argmin_rows_kernel(const float* __restrict__ dist, int rows, int K,
-                                   uint32_t* __restrict__ assign) {
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (warp >= rows) return;
-    const float* r = dist + (size_t)warp * K;
-    float best = INFINITY;
-    int bi = 0x7fffffff;
-    for (int c = lane; c < K; c += 32) {
-        const float v = r[c];
-        if (v < best) {  // ascending c per lane: the first minimum stays
-            best = v;
-            bi = c;
-        }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const float ov = __shfl_xor_sync(0xffffffffu, best, o);
-        const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-        if (ov < best || (ov == best && oi < bi)) {
-            best = ov;
-            bi = oi;
-        }
-    }
-    if (lane == 0) assign[warp] = (uint32_t)(bi == 0x7fffffff ? 0 : bi);
+// assign[i] = the column of nearest[i] (0 where no column had a finite value),
+// which is made ready for the next product (all ones).
+__global__ void take_nearest_kernel(unsigned long long* __restrict__ nearest, int rows,
+                                    uint32_t* __restrict__ assign) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= rows) return;
+    const unsigned long long key = nearest[i];
+    assign[i] = key == ~0ull ? 0u : (uint32_t)key;
+    nearest[i] = ~0ull;
 }
 
 // sums[c][d] += round(x[i][d] * scale), counts[c] += 1 for c = assign[i].
