@@ -978,8 +978,7 @@ bool probe_warp_form(const ProbeArgs& a) {
     return !a.sort_global && a.K > kProbeWarpCap && msel < kProbeWarpCap;
 }
 
-// The fallback of the probe kernels: all K exact distances for the queries
-// whose cut was not proven.
+// The fallback of the probe kernels, for the queries whose cut was not proven.
 erq_status launch_probe_exact(const Batch& b, const ProbeArgs& a, int npow2, cudaStream_t st) {
     LaunchTimer t(kProbe, st);
     probe_exact_kernel<<<(unsigned)b.nq, kProbeThreads,
