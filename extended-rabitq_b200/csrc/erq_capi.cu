@@ -523,11 +523,14 @@ int device_sms() {
 template <int EX>
 erq_status configure_refine() {
     ERQ_CUDA(cudaFuncSetAttribute(refine_kernel<EX, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
+    ERQ_CUDA(cudaFuncSetAttribute(refine_kernel<EX, kMidWarps>, cudaFuncAttributeMaxDynamicSharedMemorySize, 80 * 1024));
     ERQ_CUDA(cudaFuncSetAttribute(refine_kernel<EX, kWideWarps>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   220 * 1024));
     return ERQ_OK;
 }
 static_assert(refine_smem_bytes<4>(kMaxD, kMaxTopK) <= 64 * 1024 &&
+                  refine_smem_bytes<kMidWarps>(kMaxD, kMaxTopK) <= 80 * 1024 &&
+                  refine_smem_bytes<kMidWarps>(kMaxD, 32) <= 80 * 1024 &&
                   refine_smem_bytes<kWideWarps>(kMaxD, kMaxTopK) <= 220 * 1024 &&
                   refine_smem_bytes<kWideWarps>(kMaxD, 32) <= 220 * 1024,
               "shared memory of the refinement");
@@ -1268,8 +1271,13 @@ erq_status launch_scan_mma(const erq_index* idx, const Batch& b, uint64_t nprobe
     return ERQ_OK;
 }
 
-// refine_warps: 4 or kWideTuning chooses the form; 0 takes the wide one when
-// the batch has no more queries than SMs.
+// refine_warps: kWideTuning takes the wide form, 4 the others; 0 takes the wide
+// one when the batch has no more queries than SMs.  Of the others the 8-warp
+// form runs batches that are one wave of its blocks: there it takes 0.78 to 0.96
+// of the 4-warp form's time (150 to 444 queries, 128 to 1536 dims, nprobe 2 to
+// 64).  Past that the 4-warp form's rate decides: 1.1 to 1.4 for queries that are
+// alike, 0.65 to 1.0 where a few have many times the candidates of the others,
+// which is not known before they run.
 erq_status launch_refine(const erq_index* idx, const Batch& b, uint64_t nprobe, uint64_t k,
                          uint32_t* out_ids, float* out_dists, cudaStream_t st,
                          const int* q_nprobe = nullptr, const uint32_t* order = nullptr,
@@ -1348,16 +1356,18 @@ erq_status launch_refine(const erq_index* idx, const Batch& b, uint64_t nprobe, 
     a.nprobe = (int)nprobe;
     a.k = (int)k;
     const unsigned grid = (unsigned)b.nq;
-    const bool wide = refine_warps ? refine_warps == kWideTuning : b.nq <= (uint64_t)device_sms();
+    const uint64_t sms = (uint64_t)device_sms();
+    const bool wide = refine_warps ? refine_warps == kWideTuning : b.nq <= sms;
+    const bool mid = !wide && b.nq <= sms * RefineForm<kMidWarps>::kPerSm;
     const int kpad = (a.k + 31) & ~31;
     const size_t smem = wide ? refine_smem_bytes<kWideWarps>(a.D, kpad) : refine_smem_bytes<4>(a.D, kpad);
+    const size_t smem_mid = refine_smem_bytes<kMidWarps>(a.D, kpad);
     LaunchTimer t(kRefine, st);
 #define ERQ_REFINE_CASE(X)                                                                          \
     case X:                                                                                         \
-        if (wide)                                                                                   \
-            refine_kernel<X, kWideWarps><<<grid, kWideWarps * 32, smem, st>>>(a); \
-        else                                                                                        \
-            refine_kernel<X, 4><<<grid, kRefineThreads, smem, st>>>(a);              \
+        if (wide) refine_kernel<X, kWideWarps><<<grid, kWideWarps * 32, smem, st>>>(a);             \
+        else if (mid) refine_kernel<X, kMidWarps><<<grid, kMidWarps * 32, smem_mid, st>>>(a);       \
+        else refine_kernel<X, 4><<<grid, kRefineThreads, smem, st>>>(a);                            \
         break;
     switch (idx->EX) {
         ERQ_REFINE_CASE(2)

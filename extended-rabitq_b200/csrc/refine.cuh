@@ -248,27 +248,34 @@ __device__ __forceinline__ bool unit_scales(float u) {
 }
 
 constexpr int kRefineThreads = 128;     // 4 warps per query
-// Wide form for small batches (a query per SM): more warps, longer lists.
+// Three forms by the warps of a query's block.  The 4-warp form has the best
+// rate (6 blocks an SM hide each other's replays); a query alone in its block
+// waits for every window, and windows of more clusters and candidates, computed
+// by more warps, are fewer and shorter.
+constexpr int kMidWarps = 8;
 constexpr int kWideWarps = 16;
 constexpr int kWideTuning = 32;  // erq_plan_tuning's refine_warps of the wide form
 
-// Window capacities of the two forms: listed candidates, clusters whose unit
+// Window capacities: blocks (a lane each), listed candidates, clusters whose unit
 // queries are staged at once (at most), block minima tested per thread.
 template <int WARPS>
 struct RefineForm {
-    static constexpr int kBlocks = WARPS == 4 ? 16 : 32;     // most blocks of a window (a lane each)
-    static constexpr int kEntries = WARPS == 4 ? 256 : 1024;
-    static constexpr int kSlots = WARPS == 4 ? 8 : 16;
-    static constexpr int kPerThread = WARPS == 4 ? 4 : 2;
+    static constexpr bool kNarrow = WARPS == 4, kWide = WARPS == kWideWarps;
+    static constexpr int kBlocks = kNarrow ? 16 : 32;
+    // 8 warps, 444 slots of one wave: 2,000 queries of 1536 dims at nprobe 64 take
+    // 730 us with 16 blocks and 256 candidates, 680 with 32 and 512, 668 with 384
+    static constexpr int kEntries = kNarrow ? 256 : (kWide ? 1024 : 384);
+    static constexpr int kSlots = kNarrow ? 8 : (kWide ? 16 : 12);
+    static constexpr int kPerThread = kWide ? 2 : 4;
     static constexpr int kWords = WARPS * kPerThread;  // 32 blocks each
-    static constexpr int kProbes = WARPS == 4 ? 128 : 256;  // probes whose clusters are kept
+    static constexpr int kProbes = kWide ? 256 : 128;  // probes whose clusters are kept
     // shared memory of a block: 6 blocks of the 4-warp form per SM (1,284 us of
     // learned refinement with 5, 1,191 with 6; with 8 the ring does not fit,
-    // 1,233), one of the wide form
-    static constexpr int kRoom = WARPS == 4 ? 36 * 1024 + 512 : 220 * 1024;
-    static constexpr int kPerSm = WARPS == 4 ? 6 : 1;
+    // 1,233), 3 of the 8-warp form (with 2, 4.69 ms where 3 take 4.22), one of
+    // the wide form
+    static constexpr int kRoom = kNarrow ? 36 * 1024 + 512 : (kWide ? 220 * 1024 : 73 * 1024 + 512);
+    static constexpr int kPerSm = kNarrow ? 6 : (kWide ? 1 : 3);
 };
-
 template <int WARPS>
 struct RefineShared {
     using F = RefineForm<WARPS>;
@@ -640,7 +647,7 @@ __device__ __forceinline__ void pool_out(SmallPool& sp, const Replay& w, int siz
     }
 }
 
-// One block of WARPS warps per query (4, or 16 in the wide form).  The query's
+// One block of WARPS warps per query (4, 8 or 16).  The query's
 // blocks - of all its probed clusters, in probe order - form one sequence; a
 // window is the next of them whose smallest lower bound (from the scan) is
 // below the threshold at the window's start (a block above it has no candidate
