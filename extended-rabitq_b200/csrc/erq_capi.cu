@@ -981,6 +981,19 @@ bool probe_warp_form(const ProbeArgs& a) {
     return !a.sort_global && a.K > kProbeWarpCap && msel < kProbeWarpCap;
 }
 
+// A block per query beats a warp per query while the blocks are about one wave
+// (6 to 8 of 256 threads per SM) and a query's exact distances are work enough
+// to share (nprobe x D).  Measured block / warp, 32 to 800 queries: 0.67 to 0.87
+// at nprobe x D = 3,072, 0.65 to 0.79 at 12,288, 0.33 to 0.64 from 46,080 on, but
+// 1.06 to 1.31 at 256 and 0.92 to 1.02 at 1,536 to 2,048; 1,200 queries: 1.20 at
+// 3,072, 1.16 at 7,680, 0.67 to 0.96 from 12,288 on; 1,800 and more: 0.76 to 1.8.
+// Where the keys are not staged it was not measured and the warps stay.
+bool probe_block_pays(const ProbeArgs& a) {
+    const uint64_t work = (uint64_t)a.check_rank * (uint64_t)a.D, sms = (uint64_t)device_sms();
+    if (a.near_d || !a.stage_keys) return false;  // features: the warp form is one launch of two
+    return (uint64_t)a.nq <= 6 * sms ? work >= 3072 : (uint64_t)a.nq <= 8 * sms && work >= 12288;
+}
+
 // The fallback of the probe kernels, for the queries whose cut was not proven.
 erq_status launch_probe_exact(const Batch& b, const ProbeArgs& a, int npow2, cudaStream_t st) {
     LaunchTimer t(kProbe, st);
@@ -1014,7 +1027,7 @@ erq_status launch_probe_tc(const erq_index* idx, const Batch& b, uint64_t nprobe
     ProbeArgs a;
     int npow2 = 0;
     ERQ_TRY(probe_args(idx, b, nprobe, near_d, a, npow2));
-    const bool warp_form = probe_warp_form(a);
+    const bool warp_form = probe_warp_form(a) && (split || !probe_block_pays(a));
     const bool first_of_two = warp_form && split && b.plist;
     {
         LaunchTimer t(kProbe, st);
