@@ -303,7 +303,7 @@ struct FqShared {
     uint32_t scan[kFqThreads / 32], at[kFqThreads / 32];
     double num, best, best_t;
     uint32_t den;
-    int n, overflow;
+    int n;
 };
 template <int CAP>
 __host__ __device__ constexpr size_t fq_smem_bytes(int D) {
@@ -386,7 +386,6 @@ __global__ void __launch_bounds__(kFqThreads) fast_quantize_kernel(const float* 
     }
     if (tid == 0) {
         sh.n = 0;
-        sh.overflow = 0;
         sh.best = 0.0;
         sh.best_t = 0.0;
     }
