@@ -973,7 +973,10 @@ __global__ void __launch_bounds__(WARPS * 32, RefineForm<WARPS>::kPerSm) refine_
                     const double br = __dsub_rn((double)tt, sh.ex_sub[cs]);
                     const float xy = __fmul_rn(xipn, y);
                     const float f = __fadd_rn(sqr_x, sh.sqy[cs]);
-                    sh.d[mine] = __double2float_rn(__dsub_rn((double)f, __dmul_rn((double)xy, br)));
+                    const float dist = __double2float_rn(__dsub_rn((double)f, __dmul_rn((double)xy, br)));
+                    // what is not a number (the factor of a damaged file) counts as
+                    // infinite: the pools order numbers only
+                    sh.d[mine] = dist == dist ? dist : INFINITY;
                     sh.id[mine] = vid;
                 }
             }
