@@ -611,16 +611,18 @@ __device__ __forceinline__ void replay_window(const Replay& w, SmallPool& sp, in
 #pragma unroll 1
         while (todo) {  // a block at a time
             const int b = __shfl_sync(0xffffffffu, blk, __ffs(todo) - 1);
+            const uint32_t last = sp.last<R>();
             if (b != cur) {
                 cur = b;
-                at_start = sp.last<R>();
+                at_start = last;
             }
             const bool mine = ((todo >> lane) & 1u) && blk == b;
             const bool candidate = mine && ol < at_start;
             todo &= ~__ballot_sync(0xffffffffu, mine);
             if (w.all) st_cand += __popc(__ballot_sync(0xffffffffu, candidate));
-            // a larger distance than the largest leaves the pool as it is
-            uint32_t in = __ballot_sync(0xffffffffu, candidate && od <= at_start);
+            // a larger distance than the largest leaves the pool as it is (in the
+            // block that filled it, infinite ones may be among the entries)
+            uint32_t in = __ballot_sync(0xffffffffu, candidate && od <= last);
 #pragma unroll 1
             while (in) {
                 const int src = __ffs(in) - 1;

@@ -52,3 +52,28 @@ def test_not_a_number_counts_as_infinite(tmp_path, k):
             assert np.isinf(d[i]).sum() == max(0, k - (n - len(bad_ids))), (nq, i)
     bad.free()
     idx.free()
+
+
+@pytest.mark.parametrize("k", [55, 70, 80, 90])
+def test_infinite_distances_keep_their_order(tmp_path, oracle_mod, k):
+    """Infinite distances are ordered like any others - equal ones newest first,
+    in the block that fills a pool too - as the C oracle does, bit for bit."""
+    path = os.path.join(tmp_path, "i.index")
+    sizes = [45, 20, 31]
+    idx, g, cent = _index(path, 128, sizes, 8, 4)
+    n = sum(sizes)
+    # about half of the distances infinite, half of them -infinity
+    bad, out, _ = _damaged(tmp_path, path, np.flatnonzero(np.arange(n) % 9), np.float32(-3e38))
+    o = oracle_mod.Oracle(out)
+    nq = _batches()[-1]
+    pick = torch.randint(0, len(sizes), (nq,), generator=g)
+    q = idx.rotate((cent[pick] + 2.0 * torch.randn(nq, 128, generator=g)).numpy())
+    ref = o.search(q, k, len(sizes), nthreads=8)
+    assert np.isinf(ref[1]).any()
+    for m in _batches():
+        ids, d = bad.search_batch(q[:m], k, len(sizes))
+        assert (ids == ref[0][:m]).all(), m
+        assert (d.view(np.uint32) == ref[1][:m].view(np.uint32)).all(), m
+    o.close()
+    bad.free()
+    idx.free()
