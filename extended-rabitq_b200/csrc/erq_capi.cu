@@ -540,24 +540,23 @@ int next_pow2(int x) {
     return p;
 }
 
-erq_status configure_kernels(int D, int K, int k) {
-    const int kp2 = next_pow2(K);
-
+// Every limit is that of the largest index and request: an index or plan with
+// smaller ones never lowers what another's launches and graphs need.
+erq_status configure_kernels() {
     ERQ_CUDA(cudaFuncSetAttribute(scan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)scan_smem_bytes(D)));
+                                  (int)scan_smem_bytes(kMaxD)));
     ERQ_CUDA(cudaFuncSetAttribute(probe_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)probe_smem_bytes(D, std::min(kp2, kProbeSortSmemKeys),
-                                                        K <= kProbeStageKeys ? K : 0)));
+                                  (int)probe_smem_bytes(kMaxD, kProbeSortSmemKeys, kProbeStageKeys)));
     ERQ_CUDA(cudaFuncSetAttribute(probe_exact_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)probe_exact_smem_bytes(D, std::min(kp2, kProbeSortSmemKeys))));
+                                  (int)probe_exact_smem_bytes(kMaxD, kProbeSortSmemKeys)));
     for (const void* f : {(const void*)probe_warp_kernel<0>, (const void*)probe_warp_kernel<1>,
                           (const void*)probe_warp_kernel<2>})
         ERQ_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)(kProbeWarpWarps * probe_warp_smem_per_warp(D))));
+                                      (int)(kProbeWarpWarps * probe_warp_smem_per_warp(kMaxD))));
     ERQ_CUDA(cudaFuncSetAttribute(scan_lowacc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)low_scan_smem_bytes(D)));
+                                  (int)low_scan_smem_bytes(kMaxD)));
     {
-        const int smem = (int)(kLowRefineWarps * low_refine_smem_per_warp(D, kMaxTopK));
+        const int smem = (int)(kLowRefineWarps * low_refine_smem_per_warp(kMaxD, kMaxTopK));
         ERQ_CUDA(cudaFuncSetAttribute(refine_lowacc_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
         ERQ_CUDA(cudaFuncSetAttribute(refine_lowacc_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
         ERQ_CUDA(cudaFuncSetAttribute(refine_lowacc_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
@@ -1429,7 +1428,7 @@ erq_status check_search_args(const erq_index* idx, uint64_t nq, uint64_t k, uint
 // Rotated queries on the device -> ids/dists on the device.
 erq_status search_device(const erq_index* idx, const float* qrot_dev, uint64_t nq, uint64_t k,
                          uint64_t nprobe, uint32_t* ids_dev, float* dists_dev, cudaStream_t st) {
-    ERQ_TRY(configure_kernels((int)idx->D, (int)idx->K, (int)k));
+    ERQ_TRY(configure_kernels());
     const uint64_t bq = batch_queries(idx, nprobe, nq);
     Scratch s(st, idx->pool);
     Batch b;
@@ -2085,7 +2084,7 @@ erq_status erq_search_noalloc(const erq_index* idx, const float* rotated_queries
     }
     uint8_t* base = nullptr;
     ERQ_TRY(noalloc_scratch(idx->device, &base));
-    ERQ_TRY(configure_kernels((int)idx->D, (int)idx->K, (int)k));
+    ERQ_TRY(configure_kernels());
     // Carve the batch buffers.  Every element a kernel reads is written
     // earlier in the same call, so nothing needs clearing between calls.
     const uint64_t np = nq * nprobe;
@@ -2123,7 +2122,7 @@ erq_status erq_debug_probe(const erq_index* idx, const float* qrot, uint64_t nq,
     if (nq == 0) return ERQ_OK;
     DeviceGuard guard;
     ERQ_TRY(guard.set(idx->device));
-    ERQ_TRY(configure_kernels((int)idx->D, (int)idx->K, 1));
+    ERQ_TRY(configure_kernels());
     cudaStream_t st = 0;
     Scratch s(st, idx->pool);
     float* q = nullptr;
@@ -2181,7 +2180,7 @@ erq_status erq_debug_scan(const erq_index* idx, const float* qrot, uint64_t nq, 
                     (unsigned long long)s_capacity, (unsigned long long)need);
     DeviceGuard guard;
     ERQ_TRY(guard.set(idx->device));
-    ERQ_TRY(configure_kernels((int)idx->D, (int)idx->K, 1));
+    ERQ_TRY(configure_kernels());
     cudaStream_t st = 0;
     Scratch s(st, idx->pool);
     float* q = nullptr;
@@ -2212,7 +2211,7 @@ erq_status erq_probe_features(const erq_index* idx, const float* rotated_queries
     if (nq == 0) return ERQ_OK;
     DeviceGuard guard;
     ERQ_TRY(guard.set(idx->device));
-    ERQ_TRY(configure_kernels((int)idx->D, (int)idx->K, 1));
+    ERQ_TRY(configure_kernels());
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const bool q_dev = is_device_ptr(rotated_queries), f_dev = is_device_ptr(features);
     Scratch s(st, idx->pool);
@@ -2499,7 +2498,7 @@ static erq_status search_learned_entry(const erq_index* idx, const erq_probe_mod
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const uint64_t nprobe_max =
         std::min<uint64_t>(idx->K, std::max<uint64_t>(nprobe_fallback, (uint64_t)m->bins[kMlpBins - 1]));
-    ERQ_TRY(configure_kernels((int)idx->D, (int)idx->K, (int)k));
+    ERQ_TRY(configure_kernels());
     const bool q_dev = is_device_ptr(rotated_queries), ids_dev = is_device_ptr(ids);
     const bool d_dev = dists == nullptr || is_device_ptr(dists);
     const bool u_dev = nprobe_used == nullptr || is_device_ptr(nprobe_used);
@@ -3075,7 +3074,11 @@ erq_status scan_batched_configure(int D, int* per_sm) {
     ERQ_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     return with_scan_batched<QB, W>(D, [&](auto kern, size_t smem) -> erq_status {
         if (smem > (size_t)optin) return ERQ_OK;
-        ERQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        // the limit of every D that shares the kernel (see configure_kernels)
+        const int top = QB == 1 || D > 1536 ? kMaxD : (D > 768 ? 1536 : 768);
+        const size_t most = scan_batch_smem_bytes(QB, W, scan_qstride(D), top);
+        ERQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)std::min(most, (size_t)optin)));
         ERQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, kern, W * 32, smem));
         return ERQ_OK;
     });
@@ -3402,7 +3405,7 @@ erq_status erq_plan_create(const erq_index* idx, const erq_probe_model* model, u
                           : p->nprobe;
     p->raw = raw_queries != 0;
     ERQ_CUDA(cudaDeviceGetAttribute(&p->sms, cudaDevAttrMultiProcessorCount, idx->device));
-    ERQ_TRY(configure_kernels((int)idx->D, (int)idx->K, (int)k));
+    ERQ_TRY(configure_kernels());
     {
         const int D = (int)idx->D;
         ERQ_TRY((scan_batched_configure<1, 4>(D, &p->per_sm[0])));
