@@ -101,22 +101,32 @@ bool is_device_ptr(const void* p) {
     return attr.type == cudaMemoryTypeDevice || attr.type == cudaMemoryTypeManaged;
 }
 
+// Bytes that one search's scratch, or one plan, made by this thread may hold
+// (erq_debug_set_memory_limit; 0: no limit).
+thread_local uint64_t g_memory_limit = 0;
+bool over_memory_limit(uint64_t held, uint64_t bytes) {
+    return g_memory_limit && held + bytes > g_memory_limit;
+}
+
 // Stream-ordered scratch allocations (from the index's memory pool) released
 // on scope exit.
 struct Scratch {
     cudaStream_t stream;
     cudaMemPool_t pool;
     std::vector<void*> ptrs;
+    uint64_t held = 0;
     Scratch(cudaStream_t s, cudaMemPool_t p) : stream(s), pool(p) {}
     template <typename T>
     erq_status alloc(T** out, size_t count) {
         void* p = nullptr;
         const size_t bytes = std::max<size_t>(count * sizeof(T), 16);
-        cudaError_t e = cudaMallocFromPoolAsync(&p, bytes, pool, stream);
+        cudaError_t e = over_memory_limit(held, bytes) ? cudaErrorMemoryAllocation
+                                                       : cudaMallocFromPoolAsync(&p, bytes, pool, stream);
         if (e != cudaSuccess)
             return fail(e == cudaErrorMemoryAllocation ? ERQ_ERR_OUT_OF_MEMORY : ERQ_ERR_CUDA,
                         "cudaMallocAsync(%zu bytes) failed: %s", bytes, cudaGetErrorString(e));
         ptrs.push_back(p);
+        held += bytes;
         *out = static_cast<T*>(p);
         return ERQ_OK;
     }
@@ -807,8 +817,7 @@ uint64_t mma_rows_bytes(const erq_index* idx, uint64_t nq, uint64_t nprobe, uint
 }
 
 template <class Alloc>
-erq_status alloc_batch(Alloc& s, const erq_index* idx, uint64_t nq, uint64_t nprobe, Batch& b,
-                       uint64_t min_pairs = 0) {
+erq_status alloc_batch(Alloc& s, const erq_index* idx, uint64_t nq, uint64_t nprobe, Batch& b) {
     b.nq = nq;
     ERQ_TRY(s.alloc(&b.dist, nq * idx->K));
     ERQ_TRY(s.alloc(&b.probe_cid, nq * nprobe));
@@ -832,13 +841,21 @@ erq_status alloc_batch(Alloc& s, const erq_index* idx, uint64_t nq, uint64_t npr
     ERQ_TRY(s.alloc(&b.fb_flag, nq));
     b.sort_cap = probe_sort_cap(idx, nprobe, true);
     if (b.sort_cap) ERQ_TRY(s.alloc(&b.sortbuf, nq * b.sort_cap));
-    // last: a batch whose rows do not fit the device scans by lookups instead
+    return ERQ_OK;
+}
+
+// The rows of the tensor-core scan, once the search has everything that it
+// cannot do without: where they do not fit the device it scans by lookups.
+template <class Alloc>
+void alloc_rows(Alloc& s, const erq_index* idx, uint64_t nq, uint64_t nprobe, uint64_t min_pairs, Batch& b) {
     const uint64_t rows = mma_rows_bytes(idx, nq, nprobe, min_pairs);
-    if (rows && s.alloc(&b.qrows, rows) != ERQ_OK) {
+    if (!rows) return;
+    const std::string error = g_last_error;
+    if (s.alloc(&b.qrows, rows) != ERQ_OK) {
         b.qrows = nullptr;
         cudaGetLastError();
+        g_last_error = error;
     }
-    return ERQ_OK;
 }
 
 // Both work orders at once: (query, probe) pairs by cluster id (or by the
@@ -1432,7 +1449,8 @@ erq_status search_device(const erq_index* idx, const float* qrot_dev, uint64_t n
     const uint64_t bq = batch_queries(idx, nprobe, nq);
     Scratch s(st, idx->pool);
     Batch b;
-    ERQ_TRY(alloc_batch(s, idx, bq, nprobe, b, bq * nprobe));
+    ERQ_TRY(alloc_batch(s, idx, bq, nprobe, b));
+    alloc_rows(s, idx, bq, nprobe, bq * nprobe, b);
     for (uint64_t q0 = 0; q0 < nq; q0 += bq) {
         b.nq = std::min(bq, nq - q0);
         b.qrot = qrot_dev + q0 * idx->D;
@@ -2525,13 +2543,14 @@ static erq_status search_learned_entry(const erq_index* idx, const erq_probe_mod
     ERQ_TRY(s.alloc(&used, nq));
     const uint64_t bq = batch_queries(idx, nprobe_max, nq);
     Batch b;
-    ERQ_TRY(alloc_batch(s, idx, bq, nprobe_max, b, bq));
+    ERQ_TRY(alloc_batch(s, idx, bq, nprobe_max, b));
     ERQ_TRY(alloc_probe_lists(s, bq, b));
     float *near_d = nullptr, *feats = nullptr;
     ERQ_TRY(s.alloc(&near_d, bq * kFeatDists));
     ERQ_TRY(s.alloc(&feats, bq * kMlpIn));
     MlpWork wk;
     ERQ_TRY(mlp_alloc(s, (int)bq, false, wk));
+    alloc_rows(s, idx, bq, nprobe_max, bq, b);
     for (uint64_t q0 = 0; q0 < nq; q0 += bq) {
         b.nq = std::min(bq, nq - q0);
         b.qrot = q + q0 * idx->D;
@@ -2955,6 +2974,11 @@ erq_status erq_debug_set_gemm_wait_limit(uint32_t polls) {
     return ERQ_OK;
 }
 
+erq_status erq_debug_set_memory_limit(uint64_t bytes) {
+    g_memory_limit = bytes;
+    return ERQ_OK;
+}
+
 erq_status erq_debug_probe_fallbacks(int device, uint64_t* count, int reset) {
     if (!count) return fail(ERQ_ERR_INVALID_ARGUMENT, "count is NULL");
     DeviceGuard guard;
@@ -3024,7 +3048,7 @@ struct Arena {
     erq_status alloc(T** out, size_t count) {
         void* p = nullptr;
         const size_t b = std::max<size_t>(count * sizeof(T), 16);
-        cudaError_t e = cudaMalloc(&p, b);
+        cudaError_t e = over_memory_limit(bytes, b) ? cudaErrorMemoryAllocation : cudaMalloc(&p, b);
         if (e != cudaSuccess)
             return fail(e == cudaErrorMemoryAllocation ? ERQ_ERR_OUT_OF_MEMORY : ERQ_ERR_CUDA,
                         "cudaMalloc(%zu bytes) for a plan failed: %s", b, cudaGetErrorString(e));
@@ -3415,8 +3439,7 @@ erq_status erq_plan_create(const erq_index* idx, const erq_probe_model* model, u
         ERQ_TRY((scan_batched_configure<4, 4>(D, &p->per_sm[4])));
         ERQ_TRY((scan_batched_configure<4, 8>(D, &p->per_sm[5])));
     }
-    ERQ_TRY(alloc_batch(p->arena, idx, max_batch, p->nprobe_run, p->b,
-                        model ? max_batch : max_batch * p->nprobe_run));
+    ERQ_TRY(alloc_batch(p->arena, idx, max_batch, p->nprobe_run, p->b));
     if (model) ERQ_TRY(alloc_probe_lists(p->arena, max_batch, p->b));
     ERQ_TRY(p->arena.alloc(&p->qin, max_batch * (p->raw ? idx->DIM : idx->D)));
     ERQ_TRY(p->arena.alloc(&p->qrot, max_batch * idx->D));
@@ -3447,6 +3470,7 @@ erq_status erq_plan_create(const erq_index* idx, const erq_probe_model* model, u
                                &p->ev_comp[1], &p->ev_out[0], &p->ev_out[1]})
             ERQ_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
     }
+    alloc_rows(p->arena, idx, max_batch, p->nprobe_run, model ? max_batch : max_batch * p->nprobe_run, p->b);
     *out = p.release();
     return ERQ_OK;
 }

@@ -66,6 +66,12 @@ ERQ_API erq_status erq_debug_set_gemm_wait_limit(uint32_t polls);
 ERQ_API erq_status erq_debug_gemm_bf16(const uint16_t* A, const uint16_t* B, uint64_t M, uint64_t N,
                                        uint64_t Kd, float* C, int device);
 
+/* The most device bytes that the scratch of one search, or one plan, made by
+ * the calling thread may hold; 0 (the default) for no limit.  An allocation
+ * past it fails as a device without room does, so a test can check what is
+ * refused and what does without. */
+ERQ_API erq_status erq_debug_set_memory_limit(uint64_t bytes);
+
 /* Queries whose coarse probe could not prove its cut from the tensor-core
  * estimates and computed all K exact distances instead, since the last reset
  * (process-wide, per device). */
