@@ -782,17 +782,6 @@ uint64_t probe_sort_cap(const erq_index* idx, uint64_t nprobe, bool features) {
     return cap > kProbeSortSmemKeys ? (uint64_t)cap : 0;
 }
 
-// Largest query batch whose scan workspace fits the budget.
-uint64_t batch_queries(const erq_index* idx, uint64_t nprobe, uint64_t nq) {
-    const uint64_t per_q = 32ull * idx->top_blocks[nprobe] * sizeof(int32_t) +
-                           idx->K * sizeof(float) + nprobe * 28 + 6 * idx->D + 4 +
-                           idx->top_blocks[nprobe] * sizeof(float);
-    const uint64_t per_q_all = per_q + probe_sort_cap(idx, nprobe, true) * sizeof(uint64_t);
-    const uint64_t budget = 3ull << 30;
-    uint64_t b = std::max<uint64_t>(1, budget / std::max<uint64_t>(per_q_all, 1));
-    return std::min(b, nq);
-}
-
 // Whether a batch of at least `pairs` (query, probe) pairs scans on the tensor
 // cores (scan_mma.cuh).  Its products cost next to nothing per query, but a
 // batch pays for two more launches and the expansion of every probed block
@@ -814,6 +803,25 @@ uint64_t mma_rows_bytes(const erq_index* idx, uint64_t nq, uint64_t nprobe, uint
     if (!scan_mma_pays(idx, min_pairs) || nq * nprobe >= (1ull << 30)) return 0;
     const uint64_t bytes = 2 * nq * nprobe * mma_row_bytes((int)idx->D);
     return bytes <= std::max<uint64_t>(1ull << 30, nq * 128 * idx->top_blocks[nprobe]) ? bytes : 0;
+}
+
+// Largest query batch whose workspace fits the budget, the tensor-core scan's
+// rows included where the batch takes them (min_probes: clusters that each
+// query scans at least; 0: no scan follows).
+uint64_t batch_queries(const erq_index* idx, uint64_t nprobe, uint64_t nq, uint64_t min_probes) {
+    const uint64_t per_q = 32ull * idx->top_blocks[nprobe] * sizeof(int32_t) +
+                           idx->K * sizeof(float) + nprobe * 28 + 6 * idx->D + 4 +
+                           idx->top_blocks[nprobe] * sizeof(float);
+    const uint64_t per_q_all = per_q + probe_sort_cap(idx, nprobe, true) * sizeof(uint64_t);
+    const auto fitting = [&](uint64_t bytes) {
+        return std::min(nq, std::max<uint64_t>(1, (3ull << 30) / std::max<uint64_t>(bytes, 1)));
+    };
+    const uint64_t b = fitting(per_q_all);
+    if (mma_rows_bytes(idx, b, nprobe, b * min_probes)) {
+        const uint64_t with_rows = fitting(per_q_all + 2 * nprobe * mma_row_bytes((int)idx->D));
+        if (mma_rows_bytes(idx, with_rows, nprobe, with_rows * min_probes)) return with_rows;
+    }
+    return b;
 }
 
 template <class Alloc>
@@ -1446,7 +1454,7 @@ erq_status check_search_args(const erq_index* idx, uint64_t nq, uint64_t k, uint
 erq_status search_device(const erq_index* idx, const float* qrot_dev, uint64_t nq, uint64_t k,
                          uint64_t nprobe, uint32_t* ids_dev, float* dists_dev, cudaStream_t st) {
     ERQ_TRY(configure_kernels());
-    const uint64_t bq = batch_queries(idx, nprobe, nq);
+    const uint64_t bq = batch_queries(idx, nprobe, nq, nprobe);
     Scratch s(st, idx->pool);
     Batch b;
     ERQ_TRY(alloc_batch(s, idx, bq, nprobe, b));
@@ -2243,7 +2251,7 @@ erq_status erq_probe_features(const erq_index* idx, const float* rotated_queries
     float* fout = features;
     if (!f_dev) ERQ_TRY(s.alloc(&fout, nq * kMlpIn));
     const uint64_t nprobe = 1;
-    const uint64_t bq = batch_queries(idx, std::max<uint64_t>(nprobe, 1), nq);
+    const uint64_t bq = batch_queries(idx, nprobe, nq, 0);
     Batch b;
     ERQ_TRY(alloc_batch(s, idx, bq, nprobe, b));
     ERQ_TRY(alloc_probe_lists(s, bq, b));
@@ -2541,7 +2549,7 @@ static erq_status search_learned_entry(const erq_index* idx, const erq_probe_mod
     if (!ids_dev) ERQ_TRY(s.alloc(&ids_out, nq * k));
     if (!d_dev) ERQ_TRY(s.alloc(&d_out, nq * k));
     ERQ_TRY(s.alloc(&used, nq));
-    const uint64_t bq = batch_queries(idx, nprobe_max, nq);
+    const uint64_t bq = batch_queries(idx, nprobe_max, nq, 1);
     Batch b;
     ERQ_TRY(alloc_batch(s, idx, bq, nprobe_max, b));
     ERQ_TRY(alloc_probe_lists(s, bq, b));
