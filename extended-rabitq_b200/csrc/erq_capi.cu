@@ -3140,7 +3140,14 @@ struct erq_plan {
     float confidence = 0.9f, min_prob = 0.f;
     int sms = 148;
     int per_sm[kNumScanShapes] = {};  // resident scan blocks per SM, by kScanShapes entry
-    std::map<uint64_t, erq_plan_tuning> tunings;  // by the batch size tuned for
+    // by the batch size tuned for; what the autotuner did not time (a tile, where
+    // its batch scanned on the tensor cores) or found best as it is by default (the
+    // refinement's form) goes by the size of the batch that uses the tuning
+    struct Tuning {
+        erq_plan_tuning t;
+        bool default_tile, default_form;
+    };
+    std::map<uint64_t, Tuning> tunings;
     Arena arena;
     Batch b;
     float* qin = nullptr;       // [max_batch][DIM or D] queries as given
@@ -3202,19 +3209,28 @@ erq_plan_tuning default_tuning(uint64_t nq) {
     return t;
 }
 
+// The refine_warps that stands for the form of a batch of nq by default (the
+// 8-warp form has none of its own).
+uint32_t default_form(uint64_t nq) {
+    const uint64_t sms = (uint64_t)device_sms();
+    return nq <= sms ? kWideTuning : (nq <= sms * RefineForm<kMidWarps>::kPerSm ? 0 : 4);
+}
+
 // Tuning for a batch of nq: the one tuned for the nearest batch size (log
 // scale), else the default.
 erq_plan_tuning plan_tuning(const erq_plan* p, uint64_t nq) {
     if (p->tunings.empty()) return default_tuning(nq);
     double best = 1e300;
-    erq_plan_tuning t = p->tunings.begin()->second;
+    erq_plan::Tuning n = p->tunings.begin()->second;
     for (auto& kv : p->tunings) {
         const double d = std::fabs(std::log((double)kv.first) - std::log((double)std::max<uint64_t>(nq, 1)));
         if (d < best) {
             best = d;
-            t = kv.second;
+            n = kv.second;
         }
     }
+    erq_plan_tuning t = n.default_tile ? default_tuning(nq) : n.t;
+    t.refine_warps = n.default_form ? default_form(nq) : n.t.refine_warps;
     return t;
 }
 
@@ -3505,7 +3521,7 @@ erq_status erq_plan_set_tuning(erq_plan* p, uint64_t batch, const erq_plan_tunin
     std::lock_guard<std::mutex> g(p->mu);
     DeviceGuard guard;
     ERQ_TRY(guard.set(p->idx->device));
-    p->tunings[std::max<uint64_t>(batch, 1)] = *t;
+    p->tunings[std::max<uint64_t>(batch, 1)] = {*t, false, false};
     p->drop_graphs();
     return ERQ_OK;
 }
@@ -3535,11 +3551,11 @@ erq_status erq_plan_autotune(erq_plan* p, const float* queries, uint64_t n, int 
     }
     float best = 1e30f;
     erq_plan_tuning bt = default_tuning(n);
+    const bool mma = plan_scans_mma(p, n);  // the tile shapes are the lookup scan's
     erq_status s = ERQ_OK;
-    for (int si = 0; si < kNumScanShapes && s == ERQ_OK; ++si) {
+    for (int si = 0; si < kNumScanShapes && s == ERQ_OK && !mma; ++si) {
         const ScanShape& sh = kScanShapes[si];
         if (!p->per_sm[si]) continue;  // does not fit at this D
-        if (plan_scans_mma(p, n)) break;  // the tile shapes are the lookup scan's
         for (int cb : kChunkChoices) {
             erq_plan_tuning t = default_tuning(n);  // refinement form by batch size
             t.queries_per_item = (uint32_t)sh.qb;
@@ -3564,9 +3580,10 @@ erq_status erq_plan_autotune(erq_plan* p, const float* queries, uint64_t n, int 
         }
         if (s != ERQ_OK) break;
     }
-    // both refinement forms with the chosen tile (the auto choice is one of them)
-    for (uint32_t rw : {4u, (uint32_t)kWideTuning}) {
+    // the refinement's forms with the chosen tile: the default and the other ones
+    for (uint32_t rw : {0u, 4u, (uint32_t)kWideTuning}) {
         if (s != ERQ_OK) break;
+        if (rw && rw == default_form(n)) continue;
         erq_plan_tuning t = bt;
         t.refine_warps = rw;
         if ((s = plan_pipeline(p, n, t, st)) != ERQ_OK) break;  // warm-up
@@ -3585,12 +3602,13 @@ erq_status erq_plan_autotune(erq_plan* p, const float* queries, uint64_t n, int 
             bt = t;
         }
     }
-    if (bt.refine_warps == 0) bt.refine_warps = n <= (uint64_t)device_sms() ? kWideTuning : 4;
+    const bool by_size = bt.refine_warps == 0;
+    if (by_size) bt.refine_warps = default_form(n);
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     ERQ_TRY(s);
     ERQ_CUDA(cudaStreamSynchronize(st));
-    p->tunings[n] = bt;
+    p->tunings[n] = {bt, mma, by_size};
     p->drop_graphs();
     if (chosen) *chosen = bt;
     if (best_ms) *best_ms = best;

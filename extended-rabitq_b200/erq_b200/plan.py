@@ -2,8 +2,9 @@
 
 A plan owns the device buffers for batches of up to ``max_batch`` queries,
 captures the search of each batch size into a CUDA graph on first use and
-replays it, and scans over a (cluster x query block x cluster chunk) work list
-whose tile shape ``autotune`` picks per batch size.  Results equal
+replays it, and scans over a (cluster x query block x cluster chunk) work list:
+large batches on the tensor cores, smaller ones by table lookups whose tile
+shape ``autotune`` picks per batch size.  Results equal
 ``IVF.search_batch`` (no model) or ``learned.search_learned`` (with a model).
 """
 from __future__ import annotations
@@ -59,7 +60,8 @@ class Plan:
 
     def set_tuning(self, batch: int, queries_per_item: int, blocks_per_item: int, warps: int,
                    refine_warps: int = 0) -> None:
-        """refine_warps: 4, 32 (wide refinement form) or 0 (by batch size)."""
+        """The tile of a lookup scan (tensor-core scans have none to choose) and
+        refine_warps: 4, 32 (wide refinement form) or 0 (by batch size)."""
         t = PlanTuning(queries_per_item, blocks_per_item, warps, refine_warps)
         check(self._lib.erq_plan_set_tuning(self._h, batch, C.byref(t)))
 

@@ -157,14 +157,18 @@ ERQ_API erq_status erq_search_learned_raw(const erq_index* index, const erq_prob
  * captures the pipeline (rotation when raw_queries, coarse probe, learned
  * cut-off when a model is given, work list, scan, refinement) into a CUDA
  * graph that later searches of that size replay.  The scan runs over a work
- * list of (cluster, up to Q queries probing it, chunk of up to C 32-vector
- * blocks) items in one persistent kernel; erq_plan_autotune times the tile
- * choices on a sample batch and keeps the fastest for that batch size.
+ * list of (cluster, queries probing it, chunk of its 32-vector blocks) items in
+ * one persistent kernel: batches of 512 (query, cluster) pairs with 2^20 dims
+ * or more in all on the tensor cores (a model counts one pair per query), in
+ * items of a fixed size; smaller ones by table lookups, in items of up to Q
+ * queries and C blocks.  erq_plan_autotune times the choices on a sample batch
+ * and keeps the fastest for that batch size.
  * Calls on one plan are serialised by the plan; use one plan per stream for
  * concurrent batches. */
 typedef struct erq_plan erq_plan;
 
 typedef struct {
+    /* the tile of a lookup scan; tensor-core scans have none to choose */
     uint32_t queries_per_item;  /* Q: 1, 2 or 4 queries sharing one cluster chunk */
     uint32_t blocks_per_item;   /* C: cluster chunk, in 32-vector blocks */
     uint32_t warps;             /* warps per scan block: 4 or 8 */
@@ -185,8 +189,9 @@ ERQ_API void erq_plan_free(erq_plan* plan);
 /* Confidence and minimum probability of the learned cut-off (defaults 0.9, 0). */
 ERQ_API erq_status erq_plan_set_learned(erq_plan* plan, float confidence, float min_prob);
 /* Times every tile choice on queries[n] (host or device; best of `reps` runs
- * each), then both refinement forms with the fastest tile, and keeps the
- * fastest for batches of about n queries. */
+ * each) where they scan by lookups, then the refinement forms with the fastest
+ * tile, and keeps the fastest for batches of about n queries.  What was not
+ * timed, or is best as it is by default, goes by the size of the batch. */
 ERQ_API erq_status erq_plan_autotune(erq_plan* plan, const float* queries, uint64_t n, int reps,
                                      erq_plan_tuning* chosen, float* best_ms);
 ERQ_API erq_status erq_plan_set_tuning(erq_plan* plan, uint64_t batch, const erq_plan_tuning* tuning);
