@@ -1308,13 +1308,13 @@ erq_status launch_scan_mma(const erq_index* idx, const Batch& b, uint64_t nprobe
     return ERQ_OK;
 }
 
-// refine_warps: kWideTuning takes the wide form, 4 the others; 0 takes the wide
-// one when the batch has no more queries than SMs.  Of the others the 8-warp
-// form runs batches that are one wave of its blocks: there it takes 0.78 to 0.96
-// of the 4-warp form's time (150 to 444 queries, 128 to 1536 dims, nprobe 2 to
-// 64).  Past that the 4-warp form's rate decides: 1.1 to 1.4 for queries that are
-// alike, 0.65 to 1.0 where a few have many times the candidates of the others,
-// which is not known before they run.
+// refine_warps: kWideTuning takes the wide form, 4 the 4-warp form, 0 the one by
+// batch size: the wide form when the batch has no more queries than SMs, the
+// 8-warp form for batches that are one wave of its blocks: there it takes 0.78
+// to 0.96 of the 4-warp form's time (150 to 444 queries, 128 to 1536 dims, nprobe
+// 2 to 64).  Past that the 4-warp form's rate decides: 1.1 to 1.4 for queries that
+// are alike, 0.65 to 1.0 where a few have many times the candidates of the
+// others, which is not known before they run.
 erq_status launch_refine(const erq_index* idx, const Batch& b, uint64_t nprobe, uint64_t k,
                          uint32_t* out_ids, float* out_dists, cudaStream_t st,
                          const int* q_nprobe = nullptr, const uint32_t* order = nullptr,
@@ -1395,7 +1395,7 @@ erq_status launch_refine(const erq_index* idx, const Batch& b, uint64_t nprobe, 
     const unsigned grid = (unsigned)b.nq;
     const uint64_t sms = (uint64_t)device_sms();
     const bool wide = refine_warps ? refine_warps == kWideTuning : b.nq <= sms;
-    const bool mid = !wide && b.nq <= sms * RefineForm<kMidWarps>::kPerSm;
+    const bool mid = !wide && !refine_warps && b.nq <= sms * RefineForm<kMidWarps>::kPerSm;
     const int kpad = (a.k + 31) & ~31;
     const size_t smem = wide ? refine_smem_bytes<kWideWarps>(a.D, kpad) : refine_smem_bytes<4>(a.D, kpad);
     const size_t smem_mid = refine_smem_bytes<kMidWarps>(a.D, kpad);

@@ -172,11 +172,11 @@ typedef struct {
     uint32_t queries_per_item;  /* Q: 1, 2 or 4 queries sharing one cluster chunk */
     uint32_t blocks_per_item;   /* C: cluster chunk, in 32-vector blocks */
     uint32_t warps;             /* warps per scan block: 4 or 8 */
-    uint32_t refine_warps;      /* refinement form: 4 (a block of 4 warps per query and windows
-                                   of 16 blocks, or 8 and 32 for batches of up to 3 queries
-                                   per SM), 32 (the wide form: 16 warps, windows of 32 blocks
-                                   and 1,024 candidates), or 0 = 32 when the batch has no more
-                                   queries than SMs, else 4 */
+    uint32_t refine_warps;      /* refinement form: 4 (a block of 4 warps per query, windows of
+                                   16 blocks), 32 (the wide form: 16 warps, windows of 32
+                                   blocks and 1,024 candidates), or 0 = 32 when the batch has
+                                   no more queries than SMs, a form of 8 warps and 32 blocks
+                                   up to 3 queries per SM, else 4 */
 } erq_plan_tuning;
 
 /* model may be NULL (plain fixed-nprobe search); with a model, nprobe is the
