@@ -38,6 +38,7 @@
 #include "layout.cuh"
 #include "lowacc.cuh"
 #include "refine.cuh"
+#include "refine_cluster.cuh"
 #include "order.cuh"
 #include "scan.cuh"
 #include "scan_batch.cuh"
@@ -218,6 +219,7 @@ struct erq_index {
     uint64_t device_bytes = 0;
     std::vector<uint32_t> h_nblocks;     // per cluster
     std::vector<uint64_t> top_blocks;    // top_blocks[p] = blocks of the p largest clusters
+    double typical_blocks = 0;           // of the cluster that a block lies in, on average
     // device arrays
     float* P = nullptr;
     float* centroids = nullptr;
@@ -363,7 +365,12 @@ erq_status load_impl(const char* path, erq_index* idx) {
         std::vector<uint64_t> nbs(idx->h_nblocks.begin(), idx->h_nblocks.end());
         std::sort(nbs.begin(), nbs.end(), std::greater<uint64_t>());
         idx->top_blocks.assign(K + 1, 0);
-        for (uint64_t i = 0; i < K; ++i) idx->top_blocks[i + 1] = idx->top_blocks[i] + nbs[i];
+        double squares = 0;
+        for (uint64_t i = 0; i < K; ++i) {
+            idx->top_blocks[i + 1] = idx->top_blocks[i] + nbs[i];
+            squares += (double)nbs[i] * (double)nbs[i];
+        }
+        idx->typical_blocks = squares / (double)std::max<uint64_t>(blocks, 1);
     }
     // The remaining bytes - P, centroids, short data, long codes, factors,
     // ids - tell the two block formats apart: 1 factor per vector
@@ -536,6 +543,12 @@ erq_status configure_refine() {
     ERQ_CUDA(cudaFuncSetAttribute(refine_kernel<EX, kMidWarps>, cudaFuncAttributeMaxDynamicSharedMemorySize, 80 * 1024));
     ERQ_CUDA(cudaFuncSetAttribute(refine_kernel<EX, kWideWarps>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   220 * 1024));
+    ERQ_CUDA(cudaFuncSetAttribute(refine_cluster_kernel<EX, kClusterWarps, kClusterWindow>,
+                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)refine_cluster_smem_bytes(kMaxD, kMaxTopK, kClusterWindow)));
+    ERQ_CUDA(cudaFuncSetAttribute(refine_cluster_kernel<EX, kClusterWideWarps, kClusterWideWindow>,
+                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)refine_cluster_smem_bytes(kMaxD, kMaxTopK, kClusterWideWindow)));
     return ERQ_OK;
 }
 static_assert(refine_smem_bytes<4>(kMaxD, kMaxTopK) <= 64 * 1024 &&
@@ -1308,6 +1321,31 @@ erq_status launch_scan_mma(const erq_index* idx, const Batch& b, uint64_t nprobe
     return ERQ_OK;
 }
 
+// Whether the refinement takes its windows per cluster (refine_cluster.cuh).
+// Refinement times across clusters over times per cluster (12 indexes of 64 to
+// 1536 dims, 3,000 and 10,000 queries):
+// - pools above kSmallPool, more queries than one wave of the 4-warp form: 1.0 to
+//   1.45 from nprobe 4 on, 0.9 to 1.4 at nprobe 1 and 2 (0.7 to 1.07 for codes of less
+//   than 8 bits); with up to a wave of queries 0.8 to 1.0 for clusters of 3 blocks,
+//   1.02 to 1.1 from 6 blocks on; with one per SM (the wide forms) 0.3 to 1.0, but
+//   1.03 to 1.14 where a cluster fills a window.
+// - smaller pools, 8-bit codes up to 1,024 dims: clusters of 6 to 31 blocks 1.0 to 1.6
+//   up to nprobe 4, 0.95 to 1.1 at 8, 0.7 at 16, smaller ones the same while k is no more
+//   than a cluster's vectors, or 1.15 to 1.2 at nprobe 1 and k above 128; larger
+//   ones 0.9 to 1.06.
+// - smaller codes: 1.1 to 1.5 for k = 1 up to nprobe 2, 0.65 to 1.2 from k = 10 on.
+bool refine_by_cluster(const erq_index* idx, uint64_t nq, uint64_t nprobe, uint64_t k, bool wide, bool mid) {
+    const double blocks = idx->typical_blocks;
+    if (wide) return k > (uint64_t)kSmallPool && blocks >= 32;
+    if (mid) return false;
+    const bool waves = nq > (uint64_t)device_sms() * RefineForm<4>::kPerSm;
+    const bool bytes = ex_storage_bits((int)idx->EX) == 8;
+    if (k > (uint64_t)kSmallPool) return (waves || blocks >= 6) && (bytes || nprobe > 2);
+    if (!waves || nprobe > 4 || idx->D > 1024 || blocks >= 32) return false;
+    if (!bytes) return nprobe <= 2 && k <= 4;
+    return blocks >= 6 || k * idx->K <= idx->N || (nprobe == 1 && k > 128);
+}
+
 // refine_warps: kWideTuning takes the wide form, 4 the 4-warp form, 0 the one by
 // batch size: the wide form when the batch has no more queries than SMs, the
 // 8-warp form for batches that are one wave of its blocks: there it takes 0.78
@@ -1399,10 +1437,18 @@ erq_status launch_refine(const erq_index* idx, const Batch& b, uint64_t nprobe, 
     const int kpad = (a.k + 31) & ~31;
     const size_t smem = wide ? refine_smem_bytes<kWideWarps>(a.D, kpad) : refine_smem_bytes<4>(a.D, kpad);
     const size_t smem_mid = refine_smem_bytes<kMidWarps>(a.D, kpad);
+    const bool by_cluster = refine_by_cluster(idx, b.nq, nprobe, k, wide, mid);
+    const size_t smem_c = refine_cluster_smem_bytes(a.D, kpad, wide ? kClusterWideWindow : kClusterWindow);
     LaunchTimer t(kRefine, st);
 #define ERQ_REFINE_CASE(X)                                                                          \
     case X:                                                                                         \
-        if (wide) refine_kernel<X, kWideWarps><<<grid, kWideWarps * 32, smem, st>>>(a);             \
+        if (by_cluster && wide)                                                                     \
+            refine_cluster_kernel<X, kClusterWideWarps, kClusterWideWindow>                         \
+                <<<grid, kClusterWideWarps * 32, smem_c, st>>>(a);                                  \
+        else if (by_cluster)                                                                        \
+            refine_cluster_kernel<X, kClusterWarps, kClusterWindow>                                 \
+                <<<grid, kClusterWarps * 32, smem_c, st>>>(a);                                      \
+        else if (wide) refine_kernel<X, kWideWarps><<<grid, kWideWarps * 32, smem, st>>>(a);        \
         else if (mid) refine_kernel<X, kMidWarps><<<grid, kMidWarps * 32, smem_mid, st>>>(a);       \
         else refine_kernel<X, 4><<<grid, kRefineThreads, smem, st>>>(a);                            \
         break;
