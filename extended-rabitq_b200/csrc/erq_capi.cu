@@ -795,33 +795,48 @@ uint64_t probe_sort_cap(const erq_index* idx, uint64_t nprobe, bool features) {
     return cap > kProbeSortSmemKeys ? (uint64_t)cap : 0;
 }
 
-// Whether a batch of at least `pairs` (query, probe) pairs scans on the tensor
-// cores (scan_mma.cuh).  Its products cost next to nothing per query, but a
-// batch pays for two more launches and the expansion of every probed block
-// whatever the number of queries that share it, while the lookups' cost grows
-// with pairs x dims.  Whole searches, lookups against products, us (best of
-// 3 x 10): 1M x 1536, K 4096: 64 pairs 479 / 483, 256 pairs 568 / 537, 1,024
-// pairs 824 / 732, 16,384 pairs 3,199 / 1,362; 768 dims, Zipf, K 4096: 1,024
-// pairs 1,697 / 1,687, 4,096 pairs 2,027 / 1,992; 128 dims, K 1024: 1,024
-// pairs 156 / 170, 4,096 pairs 201 / 196, 16,384 pairs 324 / 232.
-bool scan_mma_pays(const erq_index* idx, uint64_t pairs) {
-    return idx->factors == 1 && pairs >= 512 && pairs * idx->D >= (1ull << 20);
+// What a batch's scan is for (none: no scan follows).
+enum class ScanFor { kNone, kSearch, kPlan, kLearned };
+
+// Pairs that a batch has at least: a learned one's depths are not known yet.
+uint64_t least_pairs(uint64_t nq, uint64_t nprobe, ScanFor what) {
+    return what == ScanFor::kLearned ? nq : nq * nprobe;
+}
+
+// Whether a batch scans on the tensor cores (scan_mma.cuh).  Its products cost
+// next to nothing per query, but a batch pays for two more launches and the
+// expansion of every probed block whatever the number of queries that share it,
+// while the lookups' cost grows with the pairs and their blocks.  Whole searches,
+// products over lookups, at clusters of 1 / 3 / 8 / 32 even blocks (256 to 1536 dims,
+// nprobe 1 to 64): 1,024 pairs 1.2 / 1.15 / 1.1 / 1.0, 2,048 pairs 1.17 / 1.1 / 1.0 / 0.85,
+// 4,096 pairs 1.06 / 0.97 / 0.87 / 0.7, 8,192 pairs 0.94 / 0.83 / 0.75 / 0.6; 0.86 from 512
+// pairs on over Zipf clusters, whose largest a lookup block walks alone.  Plans
+// order their pairs for lookups too: 1,024 pairs 1.13 / 1.07 / 1.0 / 0.82, 2,048
+// pairs 1.09 / 1.0 / 0.92 / 0.66, and 0.8 to 0.98 for 1,024 queries and more whatever
+// the cluster (the lookups' tile is then for more queries per cluster).  Learned
+// batches have some times the pairs that are counted.
+bool scan_mma_pays(const erq_index* idx, uint64_t nq, uint64_t nprobe, ScanFor what) {
+    const uint64_t pairs = least_pairs(nq, nprobe, what);
+    if (what == ScanFor::kNone || idx->factors != 1 || pairs < 512 || pairs * idx->D < (1ull << 20)) return false;
+    if (what == ScanFor::kLearned || idx->top_blocks[1] >= 64) return true;
+    const double p = (double)pairs, blocks = idx->typical_blocks;
+    if (what == ScanFor::kPlan) return nq >= 1024 || (p - 512) * blocks >= 5000;
+    return (p - 1024) * (blocks + 1) >= 10240;
 }
 
 // Bytes of the quantized rows of nq * nprobe pairs, 0 when they are not kept:
-// when no batch of this size uses them (min_pairs: the pairs it has at
-// least), or when they would be more than the sums they lead to (S) and 1 GiB
-// - a very large batch over tiny clusters, which then scans by lookups.
-uint64_t mma_rows_bytes(const erq_index* idx, uint64_t nq, uint64_t nprobe, uint64_t min_pairs) {
-    if (!scan_mma_pays(idx, min_pairs) || nq * nprobe >= (1ull << 30)) return 0;
+// when no batch of this size uses them, or when they would be more than the sums
+// they lead to (S) and 1 GiB - a very large batch over tiny clusters, which then
+// scans by lookups.
+uint64_t mma_rows_bytes(const erq_index* idx, uint64_t nq, uint64_t nprobe, ScanFor what) {
+    if (!scan_mma_pays(idx, nq, nprobe, what) || nq * nprobe >= (1ull << 30)) return 0;
     const uint64_t bytes = 2 * nq * nprobe * mma_row_bytes((int)idx->D);
     return bytes <= std::max<uint64_t>(1ull << 30, nq * 128 * idx->top_blocks[nprobe]) ? bytes : 0;
 }
 
-// Largest query batch whose workspace fits the budget, the tensor-core scan's
-// rows included where the batch takes them (min_probes: clusters that each
-// query scans at least; 0: no scan follows).
-uint64_t batch_queries(const erq_index* idx, uint64_t nprobe, uint64_t nq, uint64_t min_probes) {
+// Largest query batch whose workspace fits the budget, the tensor-core scan's rows
+// included where the batch takes them.
+uint64_t batch_queries(const erq_index* idx, uint64_t nprobe, uint64_t nq, ScanFor what) {
     const uint64_t per_q = 32ull * idx->top_blocks[nprobe] * sizeof(int32_t) +
                            idx->K * sizeof(float) + nprobe * 28 + 6 * idx->D + 4 +
                            idx->top_blocks[nprobe] * sizeof(float);
@@ -830,9 +845,9 @@ uint64_t batch_queries(const erq_index* idx, uint64_t nprobe, uint64_t nq, uint6
         return std::min(nq, std::max<uint64_t>(1, (3ull << 30) / std::max<uint64_t>(bytes, 1)));
     };
     const uint64_t b = fitting(per_q_all);
-    if (mma_rows_bytes(idx, b, nprobe, b * min_probes)) {
+    if (mma_rows_bytes(idx, b, nprobe, what)) {
         const uint64_t with_rows = fitting(per_q_all + 2 * nprobe * mma_row_bytes((int)idx->D));
-        if (mma_rows_bytes(idx, with_rows, nprobe, with_rows * min_probes)) return with_rows;
+        if (mma_rows_bytes(idx, with_rows, nprobe, what)) return with_rows;
     }
     return b;
 }
@@ -868,8 +883,8 @@ erq_status alloc_batch(Alloc& s, const erq_index* idx, uint64_t nq, uint64_t npr
 // The rows of the tensor-core scan, once the search has everything that it
 // cannot do without: where they do not fit the device it scans by lookups.
 template <class Alloc>
-void alloc_rows(Alloc& s, const erq_index* idx, uint64_t nq, uint64_t nprobe, uint64_t min_pairs, Batch& b) {
-    const uint64_t rows = mma_rows_bytes(idx, nq, nprobe, min_pairs);
+void alloc_rows(Alloc& s, const erq_index* idx, uint64_t nq, uint64_t nprobe, ScanFor what, Batch& b) {
+    const uint64_t rows = mma_rows_bytes(idx, nq, nprobe, what);
     if (!rows) return;
     const std::string error = g_last_error;
     if (s.alloc(&b.qrows, rows) != ERQ_OK) {
@@ -1471,7 +1486,7 @@ erq_status launch_refine(const erq_index* idx, const Batch& b, uint64_t nprobe, 
 // holds the refinement's order.
 erq_status order_and_scan(const erq_index* idx, const Batch& b, uint64_t nprobe, cudaStream_t st,
                           const int* q_nprobe, bool* ordered) {
-    if (b.qrows && scan_mma_pays(idx, q_nprobe ? b.nq : b.nq * nprobe)) {
+    if (b.qrows && scan_mma_pays(idx, b.nq, nprobe, q_nprobe ? ScanFor::kLearned : ScanFor::kSearch)) {
         ERQ_TRY(order_both(idx, b, nprobe, st, q_nprobe, false));
         *ordered = true;
         return launch_scan_mma(idx, b, nprobe, st);
@@ -1500,11 +1515,11 @@ erq_status check_search_args(const erq_index* idx, uint64_t nq, uint64_t k, uint
 erq_status search_device(const erq_index* idx, const float* qrot_dev, uint64_t nq, uint64_t k,
                          uint64_t nprobe, uint32_t* ids_dev, float* dists_dev, cudaStream_t st) {
     ERQ_TRY(configure_kernels());
-    const uint64_t bq = batch_queries(idx, nprobe, nq, nprobe);
+    const uint64_t bq = batch_queries(idx, nprobe, nq, ScanFor::kSearch);
     Scratch s(st, idx->pool);
     Batch b;
     ERQ_TRY(alloc_batch(s, idx, bq, nprobe, b));
-    alloc_rows(s, idx, bq, nprobe, bq * nprobe, b);
+    alloc_rows(s, idx, bq, nprobe, ScanFor::kSearch, b);
     for (uint64_t q0 = 0; q0 < nq; q0 += bq) {
         b.nq = std::min(bq, nq - q0);
         b.qrot = qrot_dev + q0 * idx->D;
@@ -2297,7 +2312,7 @@ erq_status erq_probe_features(const erq_index* idx, const float* rotated_queries
     float* fout = features;
     if (!f_dev) ERQ_TRY(s.alloc(&fout, nq * kMlpIn));
     const uint64_t nprobe = 1;
-    const uint64_t bq = batch_queries(idx, nprobe, nq, 0);
+    const uint64_t bq = batch_queries(idx, nprobe, nq, ScanFor::kNone);
     Batch b;
     ERQ_TRY(alloc_batch(s, idx, bq, nprobe, b));
     ERQ_TRY(alloc_probe_lists(s, bq, b));
@@ -2595,7 +2610,7 @@ static erq_status search_learned_entry(const erq_index* idx, const erq_probe_mod
     if (!ids_dev) ERQ_TRY(s.alloc(&ids_out, nq * k));
     if (!d_dev) ERQ_TRY(s.alloc(&d_out, nq * k));
     ERQ_TRY(s.alloc(&used, nq));
-    const uint64_t bq = batch_queries(idx, nprobe_max, nq, 1);
+    const uint64_t bq = batch_queries(idx, nprobe_max, nq, ScanFor::kLearned);
     Batch b;
     ERQ_TRY(alloc_batch(s, idx, bq, nprobe_max, b));
     ERQ_TRY(alloc_probe_lists(s, bq, b));
@@ -2604,7 +2619,7 @@ static erq_status search_learned_entry(const erq_index* idx, const erq_probe_mod
     ERQ_TRY(s.alloc(&feats, bq * kMlpIn));
     MlpWork wk;
     ERQ_TRY(mlp_alloc(s, (int)bq, false, wk));
-    alloc_rows(s, idx, bq, nprobe_max, bq, b);
+    alloc_rows(s, idx, bq, nprobe_max, ScanFor::kLearned, b);
     for (uint64_t q0 = 0; q0 < nq; q0 += bq) {
         b.nq = std::min(bq, nq - q0);
         b.qrot = q + q0 * idx->D;
@@ -3287,10 +3302,10 @@ bool tuning_valid(const erq_plan_tuning& t) {
            (t.refine_warps == 0 || t.refine_warps == 4 || t.refine_warps == (uint32_t)kWideTuning);
 }
 
-// Whether the plan's batches of nq queries scan on the tensor cores (a learned
-// plan counts one pair per query, the least it can have).
+ScanFor plan_scan(const erq_plan* p) { return p->model ? ScanFor::kLearned : ScanFor::kPlan; }
+// Whether the plan's batches of nq queries scan on the tensor cores.
 bool plan_scans_mma(const erq_plan* p, uint64_t nq) {
-    return p->b.qrows && scan_mma_pays(p->idx, p->model ? nq : nq * p->nprobe_run);
+    return p->b.qrows && scan_mma_pays(p->idx, nq, p->nprobe_run, plan_scan(p));
 }
 
 erq_status launch_scan_batched(erq_plan* p, const erq_plan_tuning& t, cudaStream_t st) {
@@ -3540,7 +3555,7 @@ erq_status erq_plan_create(const erq_index* idx, const erq_probe_model* model, u
                                &p->ev_comp[1], &p->ev_out[0], &p->ev_out[1]})
             ERQ_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
     }
-    alloc_rows(p->arena, idx, max_batch, p->nprobe_run, model ? max_batch : max_batch * p->nprobe_run, p->b);
+    alloc_rows(p->arena, idx, max_batch, p->nprobe_run, plan_scan(p.get()), p->b);
     *out = p.release();
     return ERQ_OK;
 }

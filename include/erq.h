@@ -158,10 +158,9 @@ ERQ_API erq_status erq_search_learned_raw(const erq_index* index, const erq_prob
  * cut-off when a model is given, work list, scan, refinement) into a CUDA
  * graph that later searches of that size replay.  The scan runs over a work
  * list of (cluster, queries probing it, chunk of its 32-vector blocks) items in
- * one persistent kernel: batches of 512 (query, cluster) pairs with 2^20 dims
- * or more in all on the tensor cores (a model counts one pair per query), in
- * items of a fixed size; smaller ones by table lookups, in items of up to Q
- * queries and C blocks.  erq_plan_autotune times the choices on a sample batch
+ * one persistent kernel: large batches (by queries, pairs, dims and the size of
+ * the clusters) on the tensor cores, in items of a fixed size; smaller ones by
+ * table lookups, in items of up to Q queries and C blocks.  erq_plan_autotune times the choices on a sample batch
  * and keeps the fastest for that batch size.
  * Calls on one plan are serialised by the plan; use one plan per stream for
  * concurrent batches. */
