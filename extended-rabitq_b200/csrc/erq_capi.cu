@@ -1349,14 +1349,20 @@ erq_status launch_scan_mma(const erq_index* idx, const Batch& b, uint64_t nprobe
 //   than a cluster's vectors, or 1.15 to 1.2 at nprobe 1 and k above 128; larger
 //   ones 0.9 to 1.06.
 // - smaller codes: 1.1 to 1.5 for k = 1 up to nprobe 2, 0.65 to 1.2 from k = 10 on.
+// - batches that are one wave here and two across clusters (6 to 8 queries per SM):
+//   1.12 to 1.5 up to nprobe 4 for 8-bit codes of any length, 1.0 to 1.3 up to nprobe 2
+//   for smaller ones.
 bool refine_by_cluster(const erq_index* idx, uint64_t nq, uint64_t nprobe, uint64_t k, bool wide, bool mid) {
     const double blocks = idx->typical_blocks;
     if (wide) return k > (uint64_t)kSmallPool && blocks >= 32;
     if (mid) return false;
-    const bool waves = nq > (uint64_t)device_sms() * RefineForm<4>::kPerSm;
+    const uint64_t sms = (uint64_t)device_sms();
+    const bool waves = nq > sms * RefineForm<4>::kPerSm;
     const bool bytes = ex_storage_bits((int)idx->EX) == 8;
     if (k > (uint64_t)kSmallPool) return (waves || blocks >= 6) && (bytes || nprobe > 2);
-    if (!waves || nprobe > 4 || idx->D > 1024 || blocks >= 32) return false;
+    if (!waves || nprobe > 4 || blocks >= 32) return false;
+    if (nq <= sms * kClusterPerSm) return bytes || nprobe <= 2;
+    if (idx->D > 1024) return false;
     if (!bytes) return nprobe <= 2 && k <= 4;
     return blocks >= 6 || k * idx->K <= idx->N || (nprobe == 1 && k > 128);
 }

@@ -19,6 +19,7 @@
 namespace erq {
 
 constexpr int kClusterWarps = 4;
+constexpr int kClusterPerSm = 8;         // blocks of the 4-warp form an SM holds
 constexpr int kClusterWindow = 16;       // blocks whose candidates are refined together
 constexpr int kClusterFirstWindow = 8;   // the same in the query's first probed cluster
 // Wide form for small batches (a query per SM): more warps, longer windows.
@@ -42,7 +43,8 @@ __host__ __device__ constexpr size_t refine_cluster_smem_bytes(int D, int kpad, 
 // each block's mask against the threshold at that block's start, the block's
 // candidates merged into the pool as inserting them in lane order would.
 template <int EX, int WARPS, int WB>
-__global__ void __launch_bounds__(WARPS * 32, WARPS == kClusterWarps ? 8 : 1) refine_cluster_kernel(RefineArgs a) {
+__global__ void __launch_bounds__(WARPS * 32, WARPS == kClusterWarps ? kClusterPerSm : 1)
+    refine_cluster_kernel(RefineArgs a) {
     constexpr int kThreads = WARPS * 32, kLanes = WB * 32;
     static_assert(WB % WARPS == 0 && kLanes <= 65536, "window lanes are listed as u16");
     extern __shared__ __align__(16) uint8_t smem_raw[];

@@ -1,8 +1,8 @@
 """The refinement with windows per cluster (csrc/refine_cluster.cuh) on both sides
 of the lines that choose it (refine_by_cluster in csrc/erq_capi.cu): pools of 256
 and 257, up to and above a wave of queries, 4 probes and 5, codes of 8 bits and
-smaller, clusters around 6 and 32 blocks, k up to a cluster's size - against the
-C oracle, ids and distance bits equal."""
+smaller, clusters around 6 and 32 blocks, k up to a cluster's size, one wave and
+more - against the C oracle, ids and distance bits equal."""
 import os
 
 import pytest
@@ -23,13 +23,13 @@ def test_windows_per_cluster(tmp_path, oracle_mod, dim, bits, sizes):
     path = os.path.join(tmp_path, "i.index")
     idx, g, cent = _index(path, dim, sizes, bits, 5 * dim + bits, dup=3)  # equal distances too
     sms = torch.cuda.get_device_properties(0).multi_processor_count
-    nq = 6 * sms + 1
+    nq = 8 * sms + 1
     pick = torch.randint(0, len(sizes), (nq,), generator=g)
     q = idx.rotate((cent[pick] + 0.7 * torch.randn(nq, dim, generator=g)).numpy())
     o = oracle_mod.Oracle(path)
     for k, nprobe in ((1, 1), (4, 2), (5, 4), (20, 4), (20, 5), (129, 1), (256, 4), (257, 4), (1024, 5)):
         ref = o.search(q, k, nprobe, nthreads=8)
-        for n in (3, 3 * sms + 1, 6 * sms, nq):
+        for n in (3, 3 * sms + 1, 6 * sms, 6 * sms + 1, 8 * sms, nq):
             _same(idx.search_batch(q[:n], k, nprobe), (ref[0][:n], ref[1][:n]))
     o.close()
     idx.free()
