@@ -1343,7 +1343,7 @@ erq_status launch_scan_mma(const erq_index* idx, const Batch& b, uint64_t nprobe
 //   1.45 from nprobe 4 on, 0.9 to 1.4 at nprobe 1 and 2 (0.7 to 1.07 for codes of less
 //   than 8 bits); with up to a wave of queries 0.8 to 1.0 for clusters of 3 blocks,
 //   1.02 to 1.1 from 6 blocks on; with one per SM (the wide forms) 0.3 to 1.0, but
-//   1.03 to 1.14 where a cluster fills a window.
+//   1.03 to 1.14 where a cluster fills a window and 1.0 to 1.13 at nprobe 1.
 // - smaller pools, 8-bit codes up to 1,024 dims: clusters of 6 to 31 blocks 1.0 to 1.6
 //   up to nprobe 4, 0.95 to 1.1 at 8, 0.7 at 16, smaller ones the same while k is no more
 //   than a cluster's vectors, or 1.15 to 1.2 at nprobe 1 and k above 128; larger
@@ -1354,7 +1354,7 @@ erq_status launch_scan_mma(const erq_index* idx, const Batch& b, uint64_t nprobe
 //   for smaller ones.
 bool refine_by_cluster(const erq_index* idx, uint64_t nq, uint64_t nprobe, uint64_t k, bool wide, bool mid) {
     const double blocks = idx->typical_blocks;
-    if (wide) return k > (uint64_t)kSmallPool && blocks >= 32;
+    if (wide) return k > (uint64_t)kSmallPool && (blocks >= 32 || nprobe == 1);
     if (mid) return false;
     const uint64_t sms = (uint64_t)device_sms();
     const bool waves = nq > sms * RefineForm<4>::kPerSm;

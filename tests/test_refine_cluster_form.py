@@ -27,7 +27,7 @@ def test_windows_per_cluster(tmp_path, oracle_mod, dim, bits, sizes):
     pick = torch.randint(0, len(sizes), (nq,), generator=g)
     q = idx.rotate((cent[pick] + 0.7 * torch.randn(nq, dim, generator=g)).numpy())
     o = oracle_mod.Oracle(path)
-    for k, nprobe in ((1, 1), (4, 2), (5, 4), (20, 4), (20, 5), (129, 1), (256, 4), (257, 4), (1024, 5)):
+    for k, nprobe in ((1, 1), (4, 2), (5, 4), (20, 4), (20, 5), (129, 1), (300, 1), (256, 4), (257, 4), (1024, 5)):
         ref = o.search(q, k, nprobe, nthreads=8)
         for n in (3, 3 * sms + 1, 6 * sms, 6 * sms + 1, 8 * sms, nq):
             _same(idx.search_batch(q[:n], k, nprobe), (ref[0][:n], ref[1][:n]))
