@@ -535,6 +535,8 @@ int device_sms() {
     return sms[dev];
 }
 
+constexpr int kMaxDevices = 64;
+
 // The limit covers every D and k, so a call never lowers it below what a
 // captured graph's launches need.
 template <int EX>
@@ -564,8 +566,16 @@ int next_pow2(int x) {
 }
 
 // Every limit is that of the largest index and request: an index or plan with
-// smaller ones never lowers what another's launches and graphs need.
+// smaller ones never lowers what another's launches and graphs need, and they are
+// set once per device (43 settings are 3 us of a call).
 erq_status configure_kernels() {
+    static std::mutex mu;
+    static bool configured[kMaxDevices] = {};
+    int dev = 0;
+    ERQ_CUDA(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= kMaxDevices) return fail(ERQ_ERR_UNSUPPORTED, "device ordinal %d", dev);
+    std::lock_guard<std::mutex> g(mu);
+    if (configured[dev]) return ERQ_OK;
     ERQ_CUDA(cudaFuncSetAttribute(scan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)scan_smem_bytes(kMaxD)));
     ERQ_CUDA(cudaFuncSetAttribute(probe_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -593,11 +603,11 @@ erq_status configure_kernels() {
     ERQ_TRY(configure_refine<6>());
     ERQ_TRY(configure_refine<7>());
     ERQ_TRY(configure_refine<8>());
+    configured[dev] = true;
     return ERQ_OK;
 }
 
 // ------------------------------------------------------------ tcgen05 GEMM
-constexpr int kMaxDevices = 64;
 // Wait status of gemm_tc_kernel (bit 0: a bounded wait ran out), one word per
 // device image of the library.
 __device__ uint32_t g_tc_status;
