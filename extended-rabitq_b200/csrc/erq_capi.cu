@@ -710,6 +710,8 @@ erq_status tensor_map_2d(CUtensorMap* m, CUtensorMapDataType type, uint64_t elt,
 // Polls per pipeline wait of the tcgen05 GEMM; lowered only by
 // erq_debug_set_gemm_wait_limit to exercise the timeout path.
 std::atomic<uint32_t> g_tc_wait_limit{kTcWaitLimit};
+// The same of scan_mma_kernel; changed only by erq_debug_set_scan_wait_limit.
+std::atomic<uint32_t> g_scan_wait_limit{kScanWaitLimit};
 
 erq_status gemm_tc(const __nv_bfloat16* A, const __nv_bfloat16* B, float* C, int M, int N, int Kd,
                    const GemmEpilogue& epi, int kernel_id, cudaStream_t st) {
@@ -1340,7 +1342,8 @@ erq_status launch_scan_mma(const erq_index* idx, const Batch& b, uint64_t nprobe
     const size_t smem = mma_smem_bytes(D);
     const int per_sm = smem <= 112 * 1024 ? 2 : 1;
     LaunchTimer t(kScan, st);
-    scan_mma_kernel<<<(unsigned)(device_sms() * per_sm), kMmaThreads, smem, st>>>(rows, (uint32_t)pairs, a);
+    scan_mma_kernel<<<(unsigned)(device_sms() * per_sm), kMmaThreads, smem, st>>>(rows, (uint32_t)pairs, a,
+                                                                               g_scan_wait_limit.load());
     t.finish();
     ERQ_CUDA(cudaGetLastError());
     return ERQ_OK;
@@ -3056,6 +3059,11 @@ erq_status erq_kmeans_step(const float* data, uint64_t n, uint64_t dim, uint64_t
 
 erq_status erq_debug_set_gemm_wait_limit(uint32_t polls) {
     g_tc_wait_limit.store(polls ? polls : kTcWaitLimit);
+    return ERQ_OK;
+}
+
+erq_status erq_debug_set_scan_wait_limit(uint32_t polls) {
+    g_scan_wait_limit.store(polls ? polls : kScanWaitLimit);
     return ERQ_OK;
 }
 

@@ -28,9 +28,11 @@
 //
 // Barriers: full/empty per ring slot, tfull/tempty per accumulator (two),
 // full/empty per record, one per K block of B, bfree when an item's products
-// are done.  Every wait is bounded; a role whose wait runs out sets the
-// block's flag and leaves, its copies and products in flight are waited for,
-// and bit kScanTimeoutBit of the status word is set.
+// are done.  Every wait is bounded (wait_limit polls); a role whose wait runs out
+// sets the block's flag and leaves, the others run out of theirs (a product warp
+// that gives up never frees B, whose copies may still be landing), copies and
+// products in flight are waited for, and bit kScanTimeoutBit of the status word
+// is set.
 #pragma once
 
 #include "common.cuh"
@@ -239,7 +241,7 @@ __device__ __forceinline__ uint32_t mma_group_start(uint32_t m, uint32_t g) {
 }
 
 __global__ void __launch_bounds__(kMmaThreads, 2)
-scan_mma_kernel(const __grid_constant__ CUtensorMap rows, uint32_t cap, ScanBatchArgs a) {
+scan_mma_kernel(const __grid_constant__ CUtensorMap rows, uint32_t cap, ScanBatchArgs a, uint32_t wait_limit) {
     extern __shared__ uint8_t smem_raw[];
     const int D = a.D;
     const int tid = threadIdx.x, lane = tid & 31;
@@ -288,7 +290,7 @@ scan_mma_kernel(const __grid_constant__ CUtensorMap rows, uint32_t cap, ScanBatc
     const uint32_t ring = tmem + 2 * kMmaAccCols;
     // the consumers' wait for item n (its record slot is n & 1); uniform
     const auto next_item = [&](uint32_t n) -> const MmaItem* {
-        if (!__all_sync(0xffffffffu, mbar_wait(rfull0 + 8 * (n & 1u), (n >> 1) & 1u, kScanWaitLimit))) {
+        if (!__all_sync(0xffffffffu, mbar_wait(rfull0 + 8 * (n & 1u), (n >> 1) & 1u, wait_limit))) {
             *flag = 1u;
             return nullptr;
         }
@@ -331,7 +333,7 @@ scan_mma_kernel(const __grid_constant__ CUtensorMap rows, uint32_t cap, ScanBatc
                     if (g0 + u < todo && ok) {
                         const uint4 w = buf[u];
                         buf[u] = load_next();
-                        ok = __all_sync(0xffffffffu, mbar_wait(empty0 + 8 * slot, phase, kScanWaitLimit));
+                        ok = __all_sync(0xffffffffu, mbar_wait(empty0 + 8 * slot, phase, wait_limit));
                         if (ok) {
                             tc_fence_after();
                             uint32_t e[kMmaChunkCols];
@@ -377,7 +379,7 @@ scan_mma_kernel(const __grid_constant__ CUtensorMap rows, uint32_t cap, ScanBatc
                 const float on = mine ? __ldg(a.onorm + (size_t)(fblock + b) * 32 + lane) : 0.f;
                 // lanes past the cluster's end get an infinite lower bound
                 const float on2 = 32 * b + lane < csize ? __fmul_rn(on, on) : INFINITY;
-                ok = __all_sync(0xffffffffu, mbar_wait(tfull0 + 8 * acc, phase, kScanWaitLimit));
+                ok = __all_sync(0xffffffffu, mbar_wait(tfull0 + 8 * acc, phase, wait_limit));
                 if (!ok) {
                     *flag = 1u;
                     break;
@@ -440,7 +442,7 @@ scan_mma_kernel(const __grid_constant__ CUtensorMap rows, uint32_t cap, ScanBatc
             const uint32_t idesc = umma_idesc_u8s8(128, (int)(2 * qp));
             const uint64_t bdesc = umma_desc_sw128(bop);
             for (uint32_t t = 0; t < tiles; ++t) {
-                ok = __all_sync(0xffffffffu, mbar_wait(tempty0 + 8 * acc, aphase, kScanWaitLimit));
+                ok = __all_sync(0xffffffffu, mbar_wait(tempty0 + 8 * acc, aphase, wait_limit));
                 if (!ok) break;
                 tc_fence_after();
                 const uint32_t d = tmem + acc * kMmaAccCols;
@@ -449,9 +451,9 @@ scan_mma_kernel(const __grid_constant__ CUtensorMap rows, uint32_t cap, ScanBatc
                     if (t == 0) {  // the K blocks of B this chunk is the first to read
                         const uint32_t f0 = (96 * k + 127) >> 7, f1 = (96 * k + 95) >> 7;
                         for (uint32_t f = f0; f <= f1 && ok; ++f)
-                            ok = __all_sync(0xffffffffu, mbar_wait(bfull0 + 8 * f, n & 1u, kScanWaitLimit));
+                            ok = __all_sync(0xffffffffu, mbar_wait(bfull0 + 8 * f, n & 1u, wait_limit));
                     }
-                    ok = ok && __all_sync(0xffffffffu, mbar_wait(full0 + 8 * slot, phase, kScanWaitLimit));
+                    ok = ok && __all_sync(0xffffffffu, mbar_wait(full0 + 8 * slot, phase, wait_limit));
                     if (!ok) break;
                     tc_fence_after();
                     if (leader) {
@@ -475,6 +477,7 @@ scan_mma_kernel(const __grid_constant__ CUtensorMap rows, uint32_t cap, ScanBatc
                 acc ^= 1u;
                 aphase ^= acc ^ 1u;
             }
+            if (!ok) break;
             if (leader) tc_commit(bfree);
         }
         if (leader && !ok) *flag = 1u;
@@ -514,7 +517,7 @@ scan_mma_kernel(const __grid_constant__ CUtensorMap rows, uint32_t cap, ScanBatc
             MmaItem* m = items + (n & 1u);
             if (n >= 2) {
                 ok = __all_sync(0xffffffffu,
-                                mbar_wait(rempty0 + 8 * (n & 1u), ((n >> 1) - 1u) & 1u, kScanWaitLimit));
+                                mbar_wait(rempty0 + 8 * (n & 1u), ((n >> 1) - 1u) & 1u, wait_limit));
                 if (!ok) break;
             }
             if (lane == 0) {
@@ -541,7 +544,7 @@ scan_mma_kernel(const __grid_constant__ CUtensorMap rows, uint32_t cap, ScanBatc
             if (it >= total) break;
             // the queries' rows, once the item before has been multiplied
             if (lane == 0) {
-                if (n >= 1) ok = mbar_wait(bfree, (n - 1u) & 1u, kScanWaitLimit);
+                if (n >= 1) ok = mbar_wait(bfree, (n - 1u) & 1u, wait_limit);
                 if (ok) {
                     const uint32_t qp = (qn + 7u) & ~7u;
                     for (uint32_t f = 0; f < nkb; ++f) {

@@ -60,6 +60,11 @@ ERQ_API erq_status erq_debug_probe_model_params(const erq_probe_model* model, fl
  * MMAs finishing) always keep the default.  Process-wide. */
 ERQ_API erq_status erq_debug_set_gemm_wait_limit(uint32_t polls);
 
+/* The same for the pipeline waits of the tensor-core scan (0 restores 2^24),
+ * whose searches then report ERQ_ERR_TIMEOUT; its drain waits keep their own
+ * limits.  A plan's graphs keep the limit they were captured with. */
+ERQ_API erq_status erq_debug_set_scan_wait_limit(uint32_t polls);
+
 /* C[M][N] = A[M][Kd] * B[N][Kd]^T on the tcgen05 GEMM of the search (BF16
  * operands given as raw 16-bit patterns, FP32 result), host buffers; Kd a
  * multiple of 64.  ERQ_ERR_TIMEOUT if one of its bounded waits ran out. */
