@@ -1917,6 +1917,16 @@ struct KmBuffers {
     }
 };
 
+// Rows split at a time: what fits the memory of 256 Mi distances (float) and the
+// splits of as many rows as those distances stand for, within the tiles that one
+// product can have.  When that is all of x it is split once, not in each iteration.
+uint64_t km_rows(uint64_t n, uint64_t dim, uint64_t k) {
+    const uint64_t Cp = (dim + 63) / 64 * 64;
+    const uint64_t rows_d = std::min<uint64_t>(n, std::max<uint64_t>(1024, (256ull << 20) / std::max<uint64_t>(k, 1)));
+    const uint64_t rows = std::max(rows_d, rows_d * (4 * k + 6 * Cp + 4) / (6 * Cp + 12));
+    return std::min<uint64_t>({n, rows, std::max<uint64_t>(1, 0x7fffffffull / div_up(k, kTcBN)) * kTcBM});
+}
+
 // Lloyd iterations (kmeans.cuh).  cent: device [k][dim], updated in place;
 // rng: the split stream; counts_host: the last iteration's cluster sizes
 // before its splits (optional); final_assign: one more assignment to the
@@ -1925,11 +1935,7 @@ erq_status km_iterate(const float* x, uint64_t n, uint64_t dim, uint64_t k, int 
                       uint32_t* assign, uint64_t& rng, uint32_t* counts_host, bool final_assign,
                       cudaStream_t st) {
     const uint64_t Cp = (dim + 63) / 64 * 64;
-    // Rows split at a time: what fits the memory of 256 Mi distances (float) and
-    // the splits of as many rows as those distances stand for.  When that is all
-    // of x it is split once, not in each iteration.
-    const uint64_t rows_d = std::min<uint64_t>(n, std::max<uint64_t>(1024, (256ull << 20) / std::max<uint64_t>(k, 1)));
-    const uint64_t R = std::min<uint64_t>(n, std::max(rows_d, rows_d * (4 * k + 6 * Cp + 4) / (6 * Cp + 12)));
+    const uint64_t R = km_rows(n, dim, k);
     KmBuffers b;
     __nv_bfloat16 *c_split = nullptr, *x_split = nullptr;
     float *cn = nullptr, *xn = nullptr;
@@ -3056,6 +3062,8 @@ erq_status erq_kmeans_step(const float* data, uint64_t n, uint64_t dim, uint64_t
     ERQ_CUDA(cudaMemcpy(counts, cnt.data(), k * sizeof(uint32_t), cudaMemcpyDefault));
     return ERQ_OK;
 }
+
+uint64_t erq_debug_kmeans_rows(uint64_t n, uint64_t dim, uint64_t k) { return km_rows(n, dim, k); }
 
 erq_status erq_debug_set_gemm_wait_limit(uint32_t polls) {
     g_tc_wait_limit.store(polls ? polls : kTcWaitLimit);

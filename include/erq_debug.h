@@ -77,6 +77,10 @@ ERQ_API erq_status erq_debug_gemm_bf16(const uint16_t* A, const uint16_t* B, uin
  * refused and what does without. */
 ERQ_API erq_status erq_debug_set_memory_limit(uint64_t bytes);
 
+/* Rows of n x dim points that k-means into k clusters takes at a time (host
+ * arithmetic, no device). */
+ERQ_API uint64_t erq_debug_kmeans_rows(uint64_t n, uint64_t dim, uint64_t k);
+
 /* Queries whose coarse probe could not prove its cut from the tensor-core
  * estimates and computed all K exact distances instead, since the last reset
  * (process-wide, per device). */
