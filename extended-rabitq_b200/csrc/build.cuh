@@ -349,7 +349,7 @@ __device__ __forceinline__ double fq_quotient(int c, double x, double y) {
 }
 
 template <int CAP>
-__global__ void __launch_bounds__(kFqThreads) fast_quantize_kernel(const float* __restrict__ xn, int rows, int D,
+__global__ void __launch_bounds__(kFqThreads) fast_quantize_kernel(const float* __restrict__ xn, int D,
                                                                    int EX, uint8_t* __restrict__ code,
                                                                    float* __restrict__ ipnorm,
                                                                    uint32_t* __restrict__ slow,

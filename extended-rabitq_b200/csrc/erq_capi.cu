@@ -774,7 +774,7 @@ struct Batch {
     uint8_t* qrows = nullptr;         // [2][nq * nprobe][mma_row_bytes] quantized pairs (scan_mma.cuh)
     uint32_t* item_off = nullptr;     // [K + 1] first work item of each cluster (scan_batch.cuh)
     uint32_t* item_counter = nullptr; // the next work item
-    uint32_t* fb_flag = nullptr;      // [nq] queries whose probe needs all K exact distances
+    uint32_t* fb_flag = nullptr;      // [nq] queries whose cut the probe could not prove
     uint64_t* sortbuf = nullptr;      // [nq][sort_cap] probe sort keys too many for shared memory
     uint64_t sort_cap = 0;
     // a split probe's sorted lists (launch_probe_tc / launch_probe_finish);
@@ -950,13 +950,13 @@ bool launch_order(const erq_index* idx, const Batch& b, uint64_t nprobe, cudaStr
 }
 
 // Candidate count for the probe: nprobe plus a margin (probe.cuh).  When the
-// margin does not prove the cut the kernel computes all K exact distances
+// margin does not prove the cut the exact distances in reach are computed
 // (counted in g_probe_fallbacks).
 int probe_candidates(uint64_t nprobe) {
     return (int)(nprobe + std::max<uint64_t>(32, nprobe / 2));
 }
 
-// Queries whose probe fell back to all K exact distances, per device image.
+// Queries whose probe fell back to the exact distances in reach, per device image.
 __device__ uint32_t g_probe_fallbacks;
 uint32_t* probe_fallback_counter() {
     static uint32_t* ptrs[kMaxDevices] = {};
@@ -2930,10 +2930,10 @@ erq_status erq_build_index(const float* data, uint64_t n, uint64_t dim, const fl
                                       (int)fq_smem_bytes<4096>(kMaxD)));
         if (fq_cap((int)D) == 2048)
             fast_quantize_kernel<2048><<<(unsigned)n, kFqThreads, fq_smem_bytes<2048>((int)D)>>>(
-                xp, (int)n, (int)D, (int)EX, code, ipn, slow, slow_n);
+                xp, (int)D, (int)EX, code, ipn, slow, slow_n);
         else
             fast_quantize_kernel<4096><<<(unsigned)n, kFqThreads, fq_smem_bytes<4096>((int)D)>>>(
-                xp, (int)n, (int)D, (int)EX, code, ipn, slow, slow_n);
+                xp, (int)D, (int)EX, code, ipn, slow, slow_n);
         ERQ_CUDA(cudaGetLastError());
         uint32_t left = 0;  // vectors the block form leaves to the serial one
         ERQ_CUDA(cudaMemcpy(&left, slow_n, sizeof(left), cudaMemcpyDeviceToHost));

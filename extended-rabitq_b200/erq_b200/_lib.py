@@ -207,7 +207,7 @@ def profile_reset() -> None:
 
 
 def probe_fallbacks(device: int = 0, reset: bool = True) -> int:
-    """Queries whose probe fell back to all K exact distances since the last reset."""
+    """Queries whose probe fell back to the exact distances in reach since the last reset."""
     n = C.c_uint64()
     check(load_library().erq_debug_probe_fallbacks(device, C.byref(n), 1 if reset else 0))
     return int(n.value)

@@ -82,7 +82,7 @@ ERQ_API erq_status erq_debug_set_memory_limit(uint64_t bytes);
 ERQ_API uint64_t erq_debug_kmeans_rows(uint64_t n, uint64_t dim, uint64_t k);
 
 /* Queries whose coarse probe could not prove its cut from the tensor-core
- * estimates and computed all K exact distances instead, since the last reset
+ * estimates and computed the exact distances in reach instead, since the last reset
  * (process-wide, per device). */
 ERQ_API erq_status erq_debug_probe_fallbacks(int device, uint64_t* count, int reset);
 
