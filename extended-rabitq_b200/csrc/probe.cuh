@@ -16,8 +16,9 @@
 //      exact top n lie in the first P: those are recomputed and sorted by
 //      (e_c, c);
 //   4. when no list position qualifies, all Msel are recomputed and the cut is
-//      checked as A - eps > e_(n); if that fails too, probe_fallback_kernel
-//      computes e_c for all K centroids and sorts them all.
+//      checked as A - eps > e_(n); if that fails too, probe_exact_kernel
+//      computes e_c for every centroid whose estimate leaves it in reach and
+//      selects among those.
 // Usually P is a few positions past n, so few centroid rows are read.
 #pragma once
 
