@@ -1309,8 +1309,9 @@ erq_status launch_scan_mma(const erq_index* idx, const Batch& b, uint64_t nprobe
         if (!configured[dev]) {  // for every D
             ERQ_CUDA(cudaFuncSetAttribute(scan_quantize_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           (int)quantize_smem_bytes(kMaxD)));
-            ERQ_CUDA(cudaFuncSetAttribute(scan_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)mma_smem_bytes(kMaxD)));
+            for (auto kernel : {scan_mma_kernel<false>, scan_mma_kernel<true>})
+                ERQ_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                              (int)mma_smem_bytes(kMaxD)));
             configured[dev] = true;
         }
     }
@@ -1342,8 +1343,9 @@ erq_status launch_scan_mma(const erq_index* idx, const Batch& b, uint64_t nprobe
     const size_t smem = mma_smem_bytes(D);
     const int per_sm = smem <= 112 * 1024 ? 2 : 1;
     LaunchTimer t(kScan, st);
-    scan_mma_kernel<<<(unsigned)(device_sms() * per_sm), kMmaThreads, smem, st>>>(rows, (uint32_t)pairs, a,
-                                                                               g_scan_wait_limit.load());
+    const uint32_t polls = g_scan_wait_limit.load();
+    const auto kernel = polls == kScanWaitLimit ? scan_mma_kernel<false> : scan_mma_kernel<true>;
+    kernel<<<(unsigned)(device_sms() * per_sm), kMmaThreads, smem, st>>>(rows, (uint32_t)pairs, a, polls);
     t.finish();
     ERQ_CUDA(cudaGetLastError());
     return ERQ_OK;

@@ -240,8 +240,12 @@ __device__ __forceinline__ uint32_t mma_group_start(uint32_t m, uint32_t g) {
     return (uint32_t)(((uint64_t)m * g) / G);
 }
 
+// LIMITED: waits give up after `polls` instead of kScanWaitLimit, which as an
+// argument costs the kernel 3 % (erq_debug_set_scan_wait_limit).
+template <bool LIMITED>
 __global__ void __launch_bounds__(kMmaThreads, 2)
-scan_mma_kernel(const __grid_constant__ CUtensorMap rows, uint32_t cap, ScanBatchArgs a, uint32_t wait_limit) {
+scan_mma_kernel(const __grid_constant__ CUtensorMap rows, uint32_t cap, ScanBatchArgs a, uint32_t polls) {
+    const uint32_t wait_limit = LIMITED ? polls : kScanWaitLimit;
     extern __shared__ uint8_t smem_raw[];
     const int D = a.D;
     const int tid = threadIdx.x, lane = tid & 31;
