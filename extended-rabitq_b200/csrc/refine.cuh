@@ -576,6 +576,7 @@ __device__ __forceinline__ void replay_window(const Replay& w, SmallPool& sp, in
     const uint32_t lt = (1u << lane) - 1u;
     int cur = -1;  // block the replay is in, and the threshold at its start
     uint32_t at_start = worst;
+    uint32_t most = worst;  // the pool's largest is no more (infinite ones may be among those that fill it)
 #pragma unroll 1
     for (int e0 = 0; e0 < w.entries; e0 += 32) {
         const int e = e0 + lane;
@@ -605,24 +606,23 @@ __device__ __forceinline__ void replay_window(const Replay& w, SmallPool& sp, in
             if (size == w.k) {
                 sp.fill<R>(w.pool_d, w.pool_id, w.k, lane, w.scratch);
                 worst = sp.last<R>();
+                most = max(most, worst);
                 todo &= __ballot_sync(0xffffffffu, w.all || od <= worst);
             }
         }
 #pragma unroll 1
         while (todo) {  // a block at a time
             const int b = __shfl_sync(0xffffffffu, blk, __ffs(todo) - 1);
-            const uint32_t last = sp.last<R>();
             if (b != cur) {
                 cur = b;
-                at_start = last;
+                at_start = most = sp.last<R>();
             }
             const bool mine = ((todo >> lane) & 1u) && blk == b;
             const bool candidate = mine && ol < at_start;
             todo &= ~__ballot_sync(0xffffffffu, mine);
             if (w.all) st_cand += __popc(__ballot_sync(0xffffffffu, candidate));
-            // a larger distance than the largest leaves the pool as it is (in the
-            // block that filled it, infinite ones may be among the entries)
-            uint32_t in = __ballot_sync(0xffffffffu, candidate && od <= last);
+            // a larger distance than the largest leaves the pool as it is
+            uint32_t in = __ballot_sync(0xffffffffu, candidate && od <= most);
 #pragma unroll 1
             while (in) {
                 const int src = __ffs(in) - 1;
@@ -975,10 +975,9 @@ __global__ void __launch_bounds__(WARPS * 32, RefineForm<WARPS>::kPerSm) refine_
                     const double br = __dsub_rn((double)tt, sh.ex_sub[cs]);
                     const float xy = __fmul_rn(xipn, y);
                     const float f = __fadd_rn(sqr_x, sh.sqy[cs]);
-                    const float dist = __double2float_rn(__dsub_rn((double)f, __dmul_rn((double)xy, br)));
                     // what is not a number (the factor of a damaged file) counts as
                     // infinite: the pools order numbers only
-                    sh.d[mine] = dist == dist ? dist : INFINITY;
+                    sh.d[mine] = fminf(__double2float_rn(__dsub_rn((double)f, __dmul_rn((double)xy, br))), INFINITY);
                     sh.id[mine] = vid;
                 }
             }

@@ -245,8 +245,8 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == kClusterWarps ? kClusterP
                         const double br = __dsub_rn((double)t, ex_sub);
                         const float xy = __fmul_rn(xipn, y);
                         const float f = __fadd_rn(sqr_x, sqy);
-                        const float dist = __double2float_rn(__dsub_rn((double)f, __dmul_rn((double)xy, br)));
-                        w_ed[slot] = dist == dist ? dist : INFINITY;  // as refine_kernel
+                        // as refine_kernel
+                        w_ed[slot] = fminf(__double2float_rn(__dsub_rn((double)f, __dmul_rn((double)xy, br))), INFINITY);
                         w_id[slot] = vid;
                     }
                     base += step;
