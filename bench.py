@@ -276,13 +276,13 @@ LEARNED_MIN_PROB = 0.25
 
 # DRAM bytes (read + write) per algorithmic byte, from one-pass ncu captures of
 # dram__bytes_read.sum + dram__bytes_write.sum on this bench's headline
-# workload, per mode and kernel (profiles/dram_traffic_sphere1536_1M_8bit.md);
-# a launch's traffic is that ratio times its algorithmic bytes.  The ratios
-# hold for the headline workload, not for other configurations.
+# workload, per mode and kernel (profiles/dram_traffic_sphere1536_1M_8bit.md).
+# The ratios hold for the headline workload, not for other configurations.
+PRODUCTS = "scan_quantize_kernel + scan_mma_kernel"
 DRAM_PER_ALGORITHMIC_BYTE = {
-    ("plain", "scan_kernel"): 0.0589, ("plain", "refine_kernel"): 0.397,
-    ("batched", "scan_batched_kernel"): 0.0587, ("batched", "refine_kernel"): 0.397,
-    ("learned", "scan_batched_kernel"): 0.260, ("learned", "refine_kernel"): 0.397,
+    ("plain", PRODUCTS): 1.373, ("plain", "refine_kernel"): 0.366,
+    ("batched", PRODUCTS): 1.365, ("batched", "refine_kernel"): 0.366,
+    ("learned", PRODUCTS): 1.533, ("learned", "refine_kernel"): 0.362,
 }
 
 
@@ -294,11 +294,30 @@ def json_peak():
         return None
 
 
-def traffic_per_launch(mode, kernel, step_bytes, launches_per_step):
+def traffic_per_step(mode, kernel, step_bytes):
     r = DRAM_PER_ALGORITHMIC_BYTE.get((mode, kernel))
-    if r is None or not launches_per_step:
-        return None
-    return int(r * step_bytes / launches_per_step)
+    return None if r is None else int(r * step_bytes)
+
+
+def scan_work(nblocks, cids, D, take=None):
+    """Algorithmic bytes per step of the scan of the probed clusters `cids`
+    (entries where `take`, if given).  "lookups": every (query, cluster) pair
+    reads the cluster's code blocks (4D bytes) and writes its sums (128 bytes a
+    block).  "products": the codes of each probed cluster once, every pair's
+    quantized rows written and read, and its sums."""
+    c = (cids if take is None else cids[take]).astype(np.int64).ravel()
+    pair_blocks = int(nblocks[c].sum())
+    row = ((D + 5) // 6 + 15) // 16 * 96
+    row = (row + 127) // 128 * 128  # bytes of the low or the high halves
+    return {"lookups": pair_blocks * (4 * D + 128),
+            "products": int(nblocks[np.unique(c)].sum()) * 4 * D + pair_blocks * 128 + c.size * 4 * row}
+
+
+def scan_kernels(mode, launches_per_step):
+    """Names of the scan's kernels and the way it counts its bytes."""
+    if launches_per_step >= 2:
+        return PRODUCTS, "products"
+    return ("scan_kernel" if mode == "plain" else "scan_batched_kernel"), "lookups"
 
 
 def reference_parity(index_path, idx, query, k, nprobe, model=None, confidence=None):
@@ -485,7 +504,6 @@ def run_ours(args, cfg, name):
     sub = min(1000, nq)
     arr = indexfile.read_index(index_path)
     nblocks = (arr.sizes.astype(np.int64) + 31) // 32
-    block_bytes = 4 * arr.D + 128
     cand_bytes = arr.D * arr.EX // 8 + 8  # EX-code row + xipnorm + id per exact candidate
     qrot_h = idx.rotate(query)
     cids, _ = idx.debug_probe(qrot_h, max(nprobe, learned.scaled_bins(nprobe, arr.K)[-1]))
@@ -519,7 +537,7 @@ def run_ours(args, cfg, name):
         ms_pe, _, _ = timed(plain_host, args.steps, args.warmup, world, stream)
         assert (ids_h.numpy().view(np.uint32) == ids0).all()
         plain["e2e"] = round(world * nq * args.steps / (ms_pe / 1e3), 1)
-    scan_bytes_plain = int(nblocks[cids[:, :nprobe].astype(np.int64)].sum()) * block_bytes
+    scan_plain = scan_work(nblocks, cids[:, :nprobe], idx.D)
 
     # --- batched plans (CUDA graphs, work-list scan, autotuned tiles)
     from erq_b200 import Plan
@@ -599,7 +617,7 @@ def run_ours(args, cfg, name):
         return ms, e2e, clocks, prof
 
     modes = {"plain": {"ms": ms_p, "prof": prof_p, "clocks": clocks_p, "recall": recall,
-                       "ids": ids0, "scan_bytes": scan_bytes_plain, "e2e_ms": ms_pe,
+                       "ids": ids0, "scan": scan_plain, "e2e_ms": ms_pe,
                        "refine_bytes": cand_plain * cand_bytes}}
     batched = None
     if not args.no_batched:
@@ -617,7 +635,7 @@ def run_ours(args, cfg, name):
             batched["e2e_one_stream"] = round(world * nq * args.steps / (plan_b.e2e_one_stream_ms / 1e3), 1)
             batched["e2e_sync"] = round(world * nq * args.steps / (plan_b.e2e_sync_ms / 1e3), 1)
         modes["batched"] = {"ms": ms_b, "prof": prof_b, "clocks": clocks_b, "recall": recall,
-                            "ids": ids0, "scan_bytes": scan_bytes_plain, "e2e_ms": e2e_b,
+                            "ids": ids0, "scan": scan_plain, "e2e_ms": e2e_b,
                             "e2e_one_stream_ms": plan_b.e2e_one_stream_ms,
                             "refine_bytes": cand_plain * cand_bytes}
         plan_b.free()
@@ -665,7 +683,7 @@ def run_ours(args, cfg, name):
             if twin_l is not None:
                 twin_l.free()
             take = np.arange(cids.shape[1])[None, :] < used.astype(np.int64)[:, None]
-            scan_bytes_l = int(nblocks[cids.astype(np.int64)][take].sum()) * block_bytes
+            scan_l = scan_work(nblocks, cids, idx.D, take)
             learned_info = {"value": round(world * nq * args.steps / (ms_l / 1e3), 1),
                             "confidence": conf, "mean_nprobe": round(float(used.mean()), 4),
                             "recall@100": round(r_l, 5),
@@ -683,7 +701,7 @@ def run_ours(args, cfg, name):
                     world * nq * args.steps / (plan_l.e2e_one_stream_ms / 1e3), 1)
                 learned_info["e2e_sync"] = round(world * nq * args.steps / (plan_l.e2e_sync_ms / 1e3), 1)
             modes["learned"] = {"ms": ms_l, "prof": prof_l, "clocks": clocks_l, "recall": r_l,
-                                "ids": ids_l, "scan_bytes": scan_bytes_l, "e2e_ms": e2e_l,
+                                "ids": ids_l, "scan": scan_l, "e2e_ms": e2e_l,
                                 "e2e_one_stream_ms": plan_l.e2e_one_stream_ms,
                                 "refine_bytes": cand_l * cand_bytes}
             learned_for_parity = (model, conf)
@@ -705,9 +723,10 @@ def run_ours(args, cfg, name):
 
             ms_d, prof_d, _ = timed(depth_step, 5, 3, world, stream)
             nl, tms = prof_d.get("scan", (0, 0.0))
-            sbytes = int(nblocks[cids_d[:, :npd].astype(np.int64)].sum()) * block_bytes
+            kernel, way = scan_kernels("plain", nl / 5)
+            sbytes = scan_work(nblocks, cids_d[:, :npd], idx.D)[way]
             ach = sbytes * 5 / (tms / 1e3) / 1e9 if tms else 0.0
-            depth_sweep.append({"nprobe": npd, "queries": nd, "kernel": "scan_kernel",
+            depth_sweep.append({"nprobe": npd, "queries": nd, "kernel": kernel,
                                 "scan_ms_per_step": round(tms / 5, 4),
                                 "scan_bytes_per_step": sbytes, "achieved_gbs": round(ach, 1),
                                 "frac": round(ach / (json_peak() or 6650.0), 4),
@@ -722,26 +741,28 @@ def run_ours(args, cfg, name):
     peak = json_peak()
     peak_src = "measured" if peak else "fallback"
     peak = peak or 6650.0
-    # algorithmic bytes per step of the two HBM-side kernels: scan = the
-    # probed clusters' code blocks (4D + 128 B per block), refine = the exact
-    # candidates' EX-code rows + xipnorm + id (D*EX/8 + 8 B each)
+    # algorithmic bytes per step: scan as scan_work counts them for the kernels
+    # that ran, refine = the exact candidates' EX-code rows + xipnorm + id
+    # (D*EX/8 + 8 B each); traffic = DRAM bytes per step
     headline = name == DEFAULT_CONFIG and not args.queries and not args.nprobe
 
     def mode_rooflines(m):
         md = modes[m]
-        names = {"scan": "scan_kernel" if m == "plain" else "scan_batched_kernel",
-                 "refine": "refine_kernel"}
         res = {}
-        for kn, step_bytes in (("scan", md["scan_bytes"]), ("refine", md["refine_bytes"])):
+        for kn in ("scan", "refine"):
             n_launch, tot_ms = md["prof"].get(kn, (0, 0.0))
             if not n_launch:
                 continue
-            achieved = step_bytes * args.steps / n_launch / (tot_ms / n_launch / 1e3) / 1e9
+            if kn == "scan":
+                kernel, way = scan_kernels(m, n_launch / args.steps)
+                step_bytes = md["scan"][way]
+            else:
+                kernel, step_bytes = "refine_kernel", md["refine_bytes"]
+            achieved = step_bytes * args.steps / (tot_ms / 1e3) / 1e9
             res[kn] = {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak,
                        "unit": "GB/s", "frac": round(achieved / peak, 4),
-                       "traffic": (traffic_per_launch(m, names[kn], step_bytes, n_launch / args.steps)
-                                   if headline else None),
-                       "kernel": names[kn], "ms_per_step": round(tot_ms / args.steps, 4),
+                       "traffic": traffic_per_step(m, kernel, step_bytes) if headline else None,
+                       "kernel": kernel, "ms_per_step": round(tot_ms / args.steps, 4),
                        "bytes_per_step": int(step_bytes),
                        "peak_source": f"{peak_src} hbm_gbs (copy)"}
         return res
@@ -785,8 +806,7 @@ def run_ours(args, cfg, name):
                        "distance_ratio": round(ratio, 5), "queries_per_step": nq,
                        "exact_probe_fallback_rate": round(fallback_rate, 5),
                        "parallelism": f"replicas x{world} (queries replicated per GPU)",
-                       "l2": "inputs larger than L2: every step streams "
-                             f"{chosen['scan_bytes'] / 1e9:.1f} GB of packed codes from a "
+                       "l2": "inputs larger than L2: every step reads the probed clusters of a "
                              f"{os.path.getsize(index_path) / 1e9:.2f} GB index"},
             "plain_gpu": plain,
             "batched_gpu": batched,
