@@ -1351,34 +1351,53 @@ erq_status launch_scan_mma(const erq_index* idx, const Batch& b, uint64_t nprobe
     return ERQ_OK;
 }
 
-// Whether the refinement takes its windows per cluster (refine_cluster.cuh).
-// Refinement times across clusters over times per cluster (12 indexes of 64 to
-// 1536 dims, 3,000 and 10,000 queries):
-// - pools above kSmallPool, more queries than one wave of the 4-warp form: 1.0 to
-//   1.45 from nprobe 4 on, 0.9 to 1.4 at nprobe 1 and 2 (0.7 to 1.07 for codes of less
-//   than 8 bits); with up to a wave of queries 0.8 to 1.0 for clusters of 3 blocks,
-//   1.02 to 1.1 from 6 blocks on; with one per SM (the wide forms) 0.3 to 1.0, but
-//   1.03 to 1.14 where a cluster fills a window and 1.0 to 1.13 at nprobe 1.
-// - smaller pools, 8-bit codes up to 1,024 dims: clusters of 6 to 31 blocks 1.0 to 1.6
-//   up to nprobe 4, 0.95 to 1.1 at 8, 0.7 at 16, smaller ones the same while k is no more
-//   than a cluster's vectors, or 1.15 to 1.2 at nprobe 1 and k above 128; larger
-//   ones 0.9 to 1.06.
-// - smaller codes: 1.1 to 1.5 for k = 1 up to nprobe 2, 0.65 to 1.2 from k = 10 on.
-// - batches that are one wave here and two across clusters (6 to 8 queries per SM):
-//   1.12 to 1.5 up to nprobe 4 for 8-bit codes of any length, 1.0 to 1.3 up to nprobe 2
-//   for smaller ones.
+// Whether the refinement takes its windows per cluster (refine_cluster.cuh).  The
+// numbers are times across clusters over times per cluster, of 20 indexes of 64 to
+// 1536 dims, 3 to 9 bits and 1 to 63 blocks per cluster, even and Zipf.
+//
+// 4 warps per query: the waves that a batch takes with 6 and with 8 blocks per SM
+// (one against two counts as 1.5) times what a block takes.  Pools above kSmallPool,
+// in batches of as many waves either way: 1.02 to 1.12 for small codes and clusters
+// of 6 blocks and more, 0.8 to 1.0 for smaller clusters; other codes 0.75 to 0.95, 0.5 to
+// 0.8 where a query's clusters are tiny or do not fill the pool; up to 512 entries at
+// nprobe 50 and more times 0.6 over clusters of a window, 0.8 over larger ones (not over
+// Zipf ones).  Smaller pools, small codes: 0.85 to 1.1 up to nprobe 4 (0.7 to 0.85 where k
+// is more than a cluster of less than 6 blocks has; 0.95 for rows of 1 KB and more), 0.6
+// to 0.9 beyond; other codes 1.1 for k up to 4 at nprobe 1 and 2, 0.5 to 0.95 else; Zipf
+// clusters 0.9, in large batches of small k 1.08 to 1.23.  One wave against two is 1.12 to
+// 1.5 up to nprobe 4.
+//
+// The wide forms, pools above kSmallPool: 1.0 to 1.13 at nprobe 1, 1.06 to 1.27 over Zipf
+// clusters while the last one probed fills most of a window, 1.02 to 1.07 up to nprobe 4
+// over clusters of 63 blocks of small codes; 0.3 to 1.0 else.
 bool refine_by_cluster(const erq_index* idx, uint64_t nq, uint64_t nprobe, uint64_t k, bool wide, bool mid) {
     const double blocks = idx->typical_blocks;
-    if (wide) return k > (uint64_t)kSmallPool && (blocks >= 32 || nprobe == 1);
-    if (mid) return false;
+    const int bits = ex_storage_bits((int)idx->EX);
+    const bool small = bits == 8 || idx->D * bits <= 256;  // a byte per code, or rows of 32 bytes
+    const bool zipf = blocks >= 128;
+    const bool large_pool = k > (uint64_t)kSmallPool;
+    if (mid || (wide && !large_pool)) return false;
+    if (wide) {
+        if (nprobe == 1) return small || blocks < 8;
+        if (zipf) return idx->top_blocks[nprobe] - idx->top_blocks[nprobe - 1] >= 24;
+        return small && blocks >= 48 && nprobe <= 4;
+    }
     const uint64_t sms = (uint64_t)device_sms();
-    const bool waves = nq > sms * RefineForm<4>::kPerSm;
-    const bool bytes = ex_storage_bits((int)idx->EX) == 8;
-    if (k > (uint64_t)kSmallPool) return (waves || blocks >= 6) && (bytes || nprobe > 2);
-    if (!waves || nprobe > 4 || blocks >= 32) return false;
-    if (nq <= sms * kClusterPerSm) return bytes || nprobe <= 2;
-    if (idx->D > 1024) return false;
-    if (!bytes) return nprobe <= 2 && k <= 4;
+    const double waves = std::min(1.5, (double)div_up(nq, sms * RefineForm<4>::kPerSm) /
+                                           (double)div_up(nq, sms * kClusterPerSm));
+    if (large_pool) {
+        double block = small ? (blocks >= 6 ? 1.05 : 0.9) : (blocks >= 3 ? 0.88 : 0.6);
+        if (nprobe == 1 && blocks < 3) block = 1.05;
+        if (nprobe == 2 && !small && blocks < 6) block = 0.6;
+        if (nprobe > 32 && k <= 512 && blocks >= 12 && !zipf) block *= blocks < 24 ? 0.6 : 0.8;
+        return block * waves > 1;
+    }
+    if (waves <= 1) return false;
+    if (zipf) return small && nq > 24 * sms && k <= 64 && nprobe <= 8;
+    if (nprobe > 4 || blocks >= 48) return false;
+    if (nq <= sms * kClusterPerSm) return small || nprobe <= 2;
+    if (idx->D > 768) return false;
+    if (!small) return nprobe <= 2 && k <= 4;
     return blocks >= 6 || k * idx->K <= idx->N || (nprobe == 1 && k > 128);
 }
 
