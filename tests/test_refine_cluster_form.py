@@ -33,3 +33,18 @@ def test_windows_per_cluster(tmp_path, oracle_mod, dim, bits, sizes):
             _same(idx.search_batch(q[:n], k, nprobe), (ref[0][:n], ref[1][:n]))
     o.close()
     idx.free()
+
+
+def test_one_cluster_of_most_blocks(tmp_path, oracle_mod):
+    """Over Zipf clusters the wide form for large pools goes by the size of the
+    last cluster probed, and large batches of small k by their queries."""
+    path = os.path.join(tmp_path, "i.index")
+    idx, g, cent = _index(path, 64, [6000, 900, 700, 40, 3], 7, 12)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    nq = 24 * sms + 1
+    q = idx.rotate((cent[torch.randint(0, 5, (nq,), generator=g)] + 0.7 * torch.randn(nq, 64, generator=g)).numpy())
+    o = oracle_mod.Oracle(path)
+    for k, nprobe, n in ((257, 1, 9), (257, 2, 9), (257, 3, 9), (300, 4, sms), (10, 1, nq), (64, 5, nq), (65, 2, nq)):
+        _same(idx.search_batch(q[:n], k, nprobe), o.search(q[:n], k, nprobe, nthreads=8))
+    o.close()
+    idx.free()
