@@ -1367,8 +1367,8 @@ erq_status launch_scan_mma(const erq_index* idx, const Batch& b, uint64_t nprobe
 // Zipf ones).  Smaller pools, small codes: 0.85 to 1.1 up to nprobe 4 (0.7 to 0.85 where k
 // is more than a cluster of less than 6 blocks has; 0.95 for rows of 1 KB and more), 0.6
 // to 0.9 beyond; other codes 1.1 for k up to 4 at nprobe 1 and 2, 0.5 to 0.95 else; Zipf
-// clusters 0.9, in large batches of small k 1.08 to 1.23.  One wave against two is 1.12 to
-// 1.5 up to nprobe 4.
+// clusters 0.6 to 0.9, in large batches of small k over the largest 1.08 to 1.23.
+// One wave against two is 1.12 to 1.5 up to nprobe 4 over even clusters.
 //
 // The wide forms, pools above kSmallPool: 1.0 to 1.13 at nprobe 1, 1.06 to 1.27 over Zipf
 // clusters while the last one probed fills most of a window, 1.02 to 1.07 up to nprobe 4
@@ -1397,8 +1397,11 @@ bool refine_by_cluster(const erq_index* idx, uint64_t nq, uint64_t nprobe, uint6
     }
     if (waves <= 1) return false;
     if (zipf) return small && nq > 24 * sms && k <= 64 && nprobe <= 8;
-    if (nprobe > 4 || blocks >= 48) return false;
-    if (nq <= sms * kClusterPerSm) return small || nprobe <= 2;
+    const double spread = blocks * (double)idx->K / (double)std::max<uint64_t>(idx->total_blocks, 1);  // 1: even
+    if (nprobe > 4 || blocks >= 48 || spread >= 4) return false;
+    if (nq <= sms * kClusterPerSm)
+        return spread < 2 && (small || nprobe <= 2) &&
+               (blocks >= 6 || 2 * k * idx->K <= 3 * idx->N || (nprobe == 1 && k > 128));
     if (idx->D > 768) return false;
     if (!small) return nprobe <= 2 && k <= 4;
     return blocks >= 6 || k * idx->K <= idx->N || (nprobe == 1 && k > 128);
