@@ -1,7 +1,7 @@
 /* CPU oracle for the Extended-RaBitQ IVF search path (test infrastructure).
  *
  * A plain-C restatement of the reference's query path, used only by the tests,
- * by __graft_entry__.smoke() and by bench.py's cpu_baseline leg as the checker.
+ * by __graft_entry__.smoke() and by bench.py's cpu_baseline leg as the CPU side.
  * It is never linked into, or called by, the product library.
  *
  * Every function cites the reference code it restates (paths relative to the
